@@ -38,6 +38,7 @@
 #include "kernels.cuh"
 #include "refine.cuh"
 #include "rowsweep.cuh"
+#include "csweep.cuh"
 #include "tsweep.cuh"
 
 using namespace wgpu;
@@ -866,7 +867,14 @@ struct within_solver {
         TsSlots ts_slots{};
         int ts_nq = 0;
         size_t ts_smem = 0;
+        // column-lane sweep (csweep.cuh): the FP64 modes of K = 2, 4, 8
+        bool cs = false;
+        CsTerms cs_terms{};
+        size_t cs_smem = 0;
     } rsw[4];
+    // the scan sweep's ranges for the FP32 normal operator where rsw is cut
+    // for the column-lane sweep (built for mixed precision only; run sums shared)
+    RowSweepK rsw_f[4];
     int* sweep_err = nullptr;   // device flag of a timed-out wait in a sweep outside the LSMR loop
     // per column bucket, the LSMR step's operator path:
     // 0 gather + full segmented-reduction scatter, 2 warp-range row sweep (rowsweep.cuh)
@@ -1068,10 +1076,10 @@ bool launch_tgather(within_solver& s, const double* x, const double* yint, doubl
 // Classifies the terms for the warp-range row sweep and builds its tables
 // (rowsweep.cuh): range bases of the run ordinals, the crossing-run fix-ups,
 // the level-sorted run combines and the remaining full-resolution terms.
+// share: only the scan sweep's ranges and partials are built (no column-lane
+// sweep, no combines), with the run sums of `share`.
 template <int K>
-within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
-    auto& rk = s.rsw[kidx(K)];
-    if (rk.ready) return rk;
+void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within_solver::RowSweepK* share) {
     const HostDesign& D = s.design;
     const uint64_t n = D.n_obs;
     Arena& A = s.arena;
@@ -1129,10 +1137,31 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
         }
     }
     rk.grid = rk.ts ? TS_GRID : rw_grid<K>();
-    const uint64_t G = (uint64_t)rk.grid * RW_WARPS;
-    const uint64_t CH = rw_chunk<K>();
+    uint64_t G = (uint64_t)rk.grid * RW_WARPS;   // ranges
+    uint64_t CH = rw_chunk<K>(), min_range = CH;
+    // several columns of an intercept-only design of at most three terms: the
+    // column-lane sweep (csweep.cuh; a third of the scan sweep's time at eight
+    // columns, half at four), one range per stream, as many blocks as the rows
+    // fill.  Slopes and more terms need loadings per row and codes of a fourth
+    // term in registers: they stay on the scan sweep.
+    if constexpr (K >= 2) {
+        if (simple && Q <= CS_MAXQ && !share) {
+            rk.cs = true;
+            int nbk = 0;
+            for (int t = 0; t < Q; ++t)
+                if (cls[t] == CLS_HIST) nbk += (int)D.terms[t].n_levels;
+            const uint64_t per_block = (uint64_t)CS_WARPS * cs_streams<K>();
+            const uint64_t want = (n + CS_MIN_RANGE * per_block - 1) / (CS_MIN_RANGE * per_block);
+            rk.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, 148ull * cs_blocks_per_sm(nbk)));
+            rk.cs_smem = cs_smem_bytes(nbk);
+            rk.cs_terms.nq = Q;
+            G = (uint64_t)rk.grid * per_block;
+            CH = CS_ROWS;
+            min_range = CS_MIN_RANGE;
+        }
+    }
     uint64_t rpr = (n + G - 1) / G;
-    rpr = std::max<uint64_t>(CH, (rpr + CH - 1) / CH * CH);
+    rpr = std::max<uint64_t>(min_range, (rpr + CH - 1) / CH * CH);
     rp.rows_per_range = (uint32_t)rpr;
     std::vector<RwFix> fixes;
     size_t first_prob = 0;
@@ -1143,6 +1172,10 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
         const size_t probs_before = first_prob;
         first_prob += (size_t)ncol;
         if (cls[t] == CLS_HIST) {
+            if (rk.cs) {
+                rk.cs_terms.cls[t] = 2;
+                rk.cs_terms.slot[t] = rp.n_buckets;
+            }
             rp.hist[rp.n_hist++] = RwHist{t, rp.n_buckets};
             rp.n_buckets += (int)(T.n_levels * ncol);
             continue;
@@ -1161,6 +1194,10 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
             });
             const bool sorted_runs = T.sorted != 0;
             const int j = rp.n_run++;
+            if (rk.cs) {
+                rk.cs_terms.cls[t] = 1;
+                rk.cs_terms.slot[t] = j;
+            }
             RwRun& rr = rp.run[j];
             rr.term = t;
             rr.direct = sorted_runs ? 1 : 0;
@@ -1188,8 +1225,9 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
             rr.tail = A.alloc<double>(G * ncol * K);
             rr.range_base = nullptr;
             rr.run_sum = nullptr;
-            if (!rr.direct) {
-                rr.range_base = A.upload(base);
+            if (!rr.direct) rr.range_base = A.upload(base);
+            if (!rr.direct && share) rr.run_sum = share->rp.run[j].run_sum;
+            if (!rr.direct && !share) {
                 rr.run_sum = A.alloc<double>(runs * ncol * K);
                 // combine: run sums grouped by level (stable in run order)
                 std::vector<uint32_t> run_level = run_levels(codes.data(), n, runs);
@@ -1214,7 +1252,7 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
             }
             continue;
         }
-        for (int c = 0; c < ncol; ++c) {
+        for (int c = 0; c < ncol && !share; ++c) {
             rk.rest_host.push_back(s.scatter_host[probs_before + c]);
             rk.rest_ptrs.push_back(s.level_ptr_host[t]);
             rk.rest_needs_rows = true;
@@ -1231,7 +1269,7 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
     bool pv;
     rk.smem = rw_smem_bytes<K, 8>(rp.n_buckets, rp.n_hist, pv);
     rk.smem_f = rw_smem_bytes<K, 4>(rp.n_buckets, rp.n_hist, pv);
-    rk.atu = A.alloc<double>(s.n_dofs * K);
+    if (!share) rk.atu = A.alloc<double>(s.n_dofs * K);
     rk.n_rest = (uint32_t)rk.rest_host.size();
     if (rk.n_rest) {
         uint64_t pos = 0, segs = 0;
@@ -1285,18 +1323,39 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
                                 for (int wtd = 0; wtd < 2; ++wtd)
                                     if (auto f = ts_kernel(mode, nq, nrun, nhist, wtd != 0))
                                         CK(cudaFuncSetAttribute(f, attr, (int)TS_SMEM_CAP));
+            } else {
+                const int cs_cap = (int)cs_smem_bytes(RW_MAX_BUCKETS);
+                CK(cudaFuncSetAttribute(k_csweep<K, 0, false>, attr, cs_cap));
+                CK(cudaFuncSetAttribute(k_csweep<K, 1, false>, attr, cs_cap));
+                CK(cudaFuncSetAttribute(k_csweep<K, 3, false>, attr, cs_cap));
+                CK(cudaFuncSetAttribute(k_csweep<K, 0, true>, attr, cs_cap));
+                CK(cudaFuncSetAttribute(k_csweep<K, 1, true>, attr, cs_cap));
+                CK(cudaFuncSetAttribute(k_csweep<K, 3, true>, attr, cs_cap));
             }
             done.emplace_back(dev, K);
         }
     }
     rk.ready = true;
+}
+
+template <int K>
+within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
+    auto& rk = s.rsw[kidx(K)];
+    if (!rk.ready) build_rowsweep<K>(s, rk, nullptr);
     return rk;
+}
+
+// the sweep plan of the FP32 normal operator
+template <int K>
+within_solver::RowSweepK& rowsweep_f(within_solver& s) {
+    return s.rsw[kidx(K)].cs ? s.rsw_f[kidx(K)] : s.rsw[kidx(K)];
 }
 
 // FP32 loading columns in the rest problems (mixed-precision inner solve)
 template <int K>
 void ensure_rowsweep_f(within_solver& s) {
     auto& rk = ensure_rowsweep<K>(s);
+    if (rk.cs && !s.rsw_f[kidx(K)].ready) build_rowsweep<K>(s, s.rsw_f[kidx(K)], &rk);
     if (rk.rest_probs_f || !rk.n_rest) return;
     std::vector<ScatterProb> pf = rk.rest_host;
     for (auto& pr : pf) {
@@ -1316,6 +1375,19 @@ void launch_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const OpPar
                      const T* rhs = nullptr, double* sq_out = nullptr, int sq_stride = 0, int* err = nullptr) {
     RwParams rp = rk.rp;
     rp.atu = atu;
+    if constexpr (K >= 2 && MODE != 2) {
+        if (rk.cs) {
+            auto sweep = op.sqrt_w ? k_csweep<K, MODE, true> : k_csweep<K, MODE, false>;
+            launch_k(sweep, rk.grid, CS_THREADS, rk.cs_smem, st, op, rp, rk.cs_terms, v, u, cur, ctl, skip, store,
+                     rhs);
+            const unsigned fb = (unsigned)(((uint64_t)rp.n_fix * K + CS_FIN_THREADS - 1) / CS_FIN_THREADS);
+            const unsigned sums = (unsigned)(K + rp.n_buckets * K), wpb = CS_FIN_THREADS / 32;
+            launch_k(k_cs_finish<K, MODE>, fb + (sums + wpb - 1) / wpb, CS_FIN_THREADS, 0, st, op, rp, rk.cs_terms,
+                     (unsigned)rk.grid, fb, cur, ctl, skip, sq_out, sq_stride);
+            g_launches += 2;
+            return;
+        }
+    }
     constexpr int BIN_BYTES = MODE == 2 ? (int)sizeof(T) : 8;
     bool priv;
     const size_t smem = rw_smem_bytes<K, BIN_BYTES>(rp.n_buckets, rp.n_hist, priv);
@@ -1739,8 +1811,8 @@ void cg_iteration(within_solver& s, within_solver::Work& w, within_solver::Mixed
     const int* skip = &m.ctl->all_done;
     if (s.path[kidx(K)] == 2) {
         auto& rk = s.rsw[kidx(K)];
-        launch_rowsweep<K, 2, float>(s, rk, s.op_f, m.q, m.p, m.t, nullptr, m.ctl, skip, rk.rest_needs_rows ? 1 : 0,
-                                     st);
+        launch_rowsweep<K, 2, float>(s, rowsweep_f<K>(s), s.op_f, m.q, m.p, m.t, nullptr, m.ctl, skip,
+                                     rk.rest_needs_rows ? 1 : 0, st);
         rowsweep_rest<K, float>(s, rk, m.t, m.q, skip, st);
     } else {
         launch_k(k_apply<K, float>, grid_for(s.n_obs, 256 * 4, 148 * 8), 256, 0, st, s.op_f, m.p, m.t, skip);
