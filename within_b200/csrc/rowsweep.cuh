@@ -742,22 +742,29 @@ __global__ void k_ptilde(uint32_t nd, const double* __restrict__ atu, double* __
     pdl_wait();
     pdl_launch_dependents();
     if (ctl->all_done) return;
-    double inv[K], coef[K];
-    bool act[K];
+    constexpr int W = fl_w<K>(), P = fl_per_row<K>();
+    const size_t total = (size_t)nd * P;
+    const size_t e0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    const int c0 = (int)(e0 % P) * W;
+    double inv[W], coef[W];
+    bool act[W], any = false;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        act[k] = !cur[k].done;
-        const double beta = cur[k].beta;
-        inv[k] = beta == 0.0 ? 0.0 : 1.0 / beta;
-        coef[k] = beta == 0.0 ? 0.0 : beta / cur[k].alpha;
+    for (int i = 0; i < W; ++i) {
+        const ColState& c = cur[c0 + i];
+        act[i] = !c.done;
+        any = any || act[i];
+        inv[i] = c.beta == 0.0 ? 0.0 : 1.0 / c.beta;
+        coef[i] = c.beta == 0.0 ? 0.0 : c.beta / c.alpha;
     }
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nd; j += gridDim.x * blockDim.x)
+    if (!any) return;
+    for (size_t e = e0; e < total; e += step) {
+        const FlVec<W> a = fl_ld<W>(atu + e * W);
+        FlVec<W> q = fl_ld<W>(pt + e * W);
 #pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (act[k]) {
-                const size_t o = (size_t)j * K + k;
-                pt[o] = atu[o] * inv[k] - coef[k] * pt[o];
-            }
+        for (int i = 0; i < W; ++i)
+            if (act[i]) q.q[i] = a.q[i] * inv[i] - coef[i] * q.q[i];
+        fl_st<W>(pt + e * W, q);
+    }
 }
 
 }  // namespace wgpu

@@ -899,6 +899,25 @@ namespace {
 
 constexpr int RED_GRID = 148 * 8;    // fixed reduction grid: deterministic partial order
 
+// Blocks of a sum over `rows` rows of K interleaved columns (fl_* kernels): four
+// accesses per thread, at most four blocks per SM.  The last block of a sum
+// waits for every block's partials and adds them, so a small vector on the full
+// grid spends its time there: k_alpha_step of eight columns took 65 us on a
+// design of 10,000 coefficients with 1184 blocks (10 us now; 37 -> 11.5 us at
+// four columns of 220,000).  A function of the design and K only: the order of
+// every sum stays fixed.
+template <int K>
+int fl_grid(uint64_t rows) {
+    return grid_for(rows * fl_per_row<K>(), RED_THREADS * 4, 148 * 4);
+}
+// Blocks of an element-wise kernel over the same rows (256 threads): with one
+// column eight blocks per SM were faster than sixteen (solution update of
+// 1,100,020 coefficients 10.0 against 11.4 us).
+template <int K>
+int fl_vec_grid(uint64_t rows) {
+    return grid_for(rows * fl_per_row<K>(), 256, K == 1 ? 148 * 8 : 148 * 16);
+}
+
 void set_device(int dev) { CK(cudaSetDevice(dev)); }
 
 // Integer passes over a column of codes on the host pool (chunks of 2^20
@@ -1528,7 +1547,7 @@ void iteration(within_solver& s, within_solver::Work& w, int par, cudaStream_t s
         auto& rk = s.rsw[kidx(K)];
         launch_rowsweep<K, 1, double>(s, rk, s.op, rk.atu, w.v, w.u, cur, w.ctl, nullptr, 0, st);
         rowsweep_rest<K, double>(s, rk, w.u, rk.atu, skip, st);
-        launch_k(k_ptilde<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, rk.atu, w.p, cur, w.ctl);
+        launch_k(k_ptilde<K>, fl_vec_grid<K>(nd), 256, 0, st, nd, rk.atu, w.p, cur, w.ctl);
         ++g_launches;
     } else {
         launch_k(k_gather_update<K>, RED_GRID, RED_THREADS, 0, st, s.op, w.v, w.u, cur, w.ctl, w.partials, w.counter);
@@ -1542,9 +1561,9 @@ void iteration(within_solver& s, within_solver::Work& w, int par, cudaStream_t s
         launch_k(k_reorth_axpy<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, j, w.ring, w.v, w.p, cur, w.ctl, w.coef);
         g_launches += 2;
     }
-    launch_k(k_alpha_step<K>, RED_GRID, RED_THREADS, 0, st, nd, w.v, w.p, cur, nxt, w.ctl, w.partials, w.counter);
+    launch_k(k_alpha_step<K>, fl_grid<K>(nd), RED_THREADS, 0, st, nd, w.v, w.p, cur, nxt, w.ctl, w.partials, w.counter);
     ++g_launches;
-    launch_k(k_solution_update<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, w.v, w.h, w.hb, w.x, nxt, w.ctl, w.ring,
+    launch_k(k_solution_update<K>, fl_vec_grid<K>(nd), 256, 0, st, nd, w.v, w.h, w.hb, w.x, nxt, w.ctl, w.ring,
                                                                       w.p);
     ++g_launches;
     (void)n;
@@ -1612,7 +1631,7 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
     const uint32_t n = (uint32_t)s.n_obs, nd = (uint32_t)s.n_dofs;
     CK(cudaMemsetAsync(w.nonfinite, 0, sizeof(int), st));
     CK(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), st));
-    launch_k(k_load_rhs<K>, RED_GRID, RED_THREADS, 0, st, n, k_used, Y, s.perm, s.op.sqrt_w, w.yint, w.b,
+    launch_k(k_load_rhs<K>, fl_grid<K>(n), RED_THREADS, 0, st, n, k_used, Y, s.perm, s.op.sqrt_w, w.yint, w.b,
                                                     w.partials, w.counter, w.bmax, w.nonfinite);
     if (ext.x0) {   // warm start: x0 into the interleaved layout (finite check)
         if (!w.x0) w.x0 = s.arena.alloc<double>(s.n_dofs * K);
@@ -1626,17 +1645,17 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
         throw WError(ERR_INVALID, ext.x0 ? "response and warm start must be finite (a non-finite value was found)"
                                          : "response must be finite (a non-finite value was found)");
     const double t_solve0 = now_s();
-    launch_k(k_norm_b<K>, RED_GRID, RED_THREADS, 0, st, n, w.b, w.bmax, w.st, tol, (long long)maxiter, k_used,
+    launch_k(k_norm_b<K>, fl_grid<K>(n), RED_THREADS, 0, st, n, w.b, w.bmax, w.st, tol, (long long)maxiter, k_used,
                                                   w.ctl, w.partials, w.counter, 0, (int)ext.stale_window,
                                                   ext.stale_threshold);
     if (ext.x0) {   // b <- b - A x0, tolerances kept relative to the original ||b||
         launch_k(k_warm_rhs<K>, RED_GRID, RED_THREADS, 0, st, s.op, w.x0, w.b, w.partials, w.counter, w.bmax);
-        launch_k(k_norm_b<K>, RED_GRID, RED_THREADS, 0, st, n, w.b, w.bmax, w.st, tol, (long long)maxiter, k_used,
+        launch_k(k_norm_b<K>, fl_grid<K>(n), RED_THREADS, 0, st, n, w.b, w.bmax, w.st, tol, (long long)maxiter, k_used,
                                                       w.ctl, w.partials, w.counter, 1, (int)ext.stale_window,
                                                       ext.stale_threshold);
         g_launches += 2;
     }
-    launch_k(k_scale_u<K>, grid_for(n, 256, 148 * 16), 256, 0, st, n, w.b, w.u, w.st);
+    launch_k(k_scale_u<K>, fl_vec_grid<K>(n), 256, 0, st, n, w.b, w.u, w.st);
     if (s.path[kidx(K)] == 2) {   // p~ = A^T u through the row sweep (adjoint mode) and its rest
         auto& rk = s.rsw[kidx(K)];
         CK(cudaMemsetAsync(w.p, 0, (size_t)nd * K * sizeof(double), st));   // levels no row reaches stay 0
@@ -1647,9 +1666,9 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
         scatter<K, 0>(s, w.u, w.p, w.st, nullptr, st);
     }
     precond_apply<K>(s, w.ctl, w.p, w.v, nullptr, st);
-    launch_k(k_alpha_init<K>, RED_GRID, RED_THREADS, 0, st, nd, w.v, w.p, w.st, w.st + 8, w.ctl, w.partials,
+    launch_k(k_alpha_init<K>, fl_grid<K>(nd), RED_THREADS, 0, st, nd, w.v, w.p, w.st, w.st + 8, w.ctl, w.partials,
                                                       w.counter);
-    launch_k(k_init_vectors<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, w.v, w.h, w.hb, w.x, w.st, w.ring, w.p);
+    launch_k(k_init_vectors<K>, fl_vec_grid<K>(nd), 256, 0, st, nd, w.v, w.h, w.hb, w.x, w.st, w.ring, w.p);
     g_launches += 6;
     Ctl ctl{};
     if (build_loop_graph<K>(s, w)) {
@@ -1962,7 +1981,7 @@ void run_mixed(within_solver& s, const double* Y, uint32_t k_used, double tol, u
     auto& m = ensure_mixed(s, K);
     const uint32_t n = (uint32_t)s.n_obs, nd = (uint32_t)s.n_dofs;
     CK(cudaMemsetAsync(w.nonfinite, 0, sizeof(int), st));
-    launch_k(k_load_rhs<K>, RED_GRID, RED_THREADS, 0, st, n, k_used, Y, s.perm, s.op.sqrt_w, w.yint, w.b, w.partials,
+    launch_k(k_load_rhs<K>, fl_grid<K>(n), RED_THREADS, 0, st, n, k_used, Y, s.perm, s.op.sqrt_w, w.yint, w.b, w.partials,
                                                     w.counter, w.bmax, w.nonfinite);
     ++g_launches;
     int nonfinite = 0;
