@@ -1,4 +1,4 @@
-// segbook.hpp -- work lists of the piece engine (seglist.cuh), built once per
+// segbook.hpp -- work lists of the list engine (seglist.cuh), built once per
 // segment pointer array on the host and shared by every column count.
 #pragma once
 #include <algorithm>
@@ -7,10 +7,13 @@
 
 namespace wgpu {
 
-// Segments of at most this many positions are summed by one group of lanes
-// each.  A longer one gives a whole warp (or several pieces) enough positions
-// to have its loads in flight at once.
+// Segments of at most SL_SHORT positions are summed by one group of lanes each,
+// longer ones of at most SL_MEDIUM by one warp, the rest in pieces by blocks.
+// SL_SHORT: one batch of loads per lane covers most of the segment.  SL_MEDIUM:
+// at eight columns a warp takes eight positions per step, so 512 positions are
+// eight batches of eight steps; a block would leave most of its warps idle.
 constexpr uint32_t SL_SHORT = 32;
+constexpr uint32_t SL_MEDIUM = 512;
 
 struct SLPiece {
     uint32_t seg, p0, p1;   // positions [p0, p1) of segment seg
@@ -18,48 +21,53 @@ struct SLPiece {
 };
 
 struct SLSplit {
-    uint32_t r0, r1;        // pieces r0..r1 (global ids), in position order
+    uint32_t r0, r1;        // pieces r0..r1, in position order
 };
 
 // One problem's share of the book: segments [first, first + n_seg).
 struct SLPart {
     uint32_t first = 0;
     uint32_t n_short = 0;
-    uint32_t ids_off = 0;       // entries of short_ids, unless every segment is short
-    bool all_short = true;      // short segment i is first + i
+    uint32_t short_off = 0;                 // entries of short_ids, unless every segment is short
+    bool all_short = true;                  // short segment i is first + i
+    uint32_t medium_lo = 0, medium_hi = 0;  // entries of medium_ids
     uint32_t piece_lo = 0, piece_hi = 0;
 };
 
 struct SegBook {
-    std::vector<uint32_t> short_ids;
+    std::vector<uint32_t> short_ids, medium_ids;
     std::vector<SLPiece> pieces;
     std::vector<SLSplit> splits;
 
     // Segment s of the problem spans ptr[s] .. ptr[s + 1], s in [first, first + n_seg).
-    // target_warps: pieces the problem's long segments are cut into, about.
-    SLPart add(const uint32_t* ptr, uint32_t first, uint32_t n_seg, uint32_t target_warps) {
+    // target_blocks: pieces the problem's long segments are cut into, about.
+    SLPart add(const uint32_t* ptr, uint32_t first, uint32_t n_seg, uint32_t target_blocks) {
         SLPart P;
         P.first = first;
-        P.ids_off = (uint32_t)short_ids.size();
-        P.piece_lo = (uint32_t)pieces.size();
+        P.short_off = (uint32_t)short_ids.size();
+        P.medium_lo = P.medium_hi = (uint32_t)medium_ids.size();
+        P.piece_lo = P.piece_hi = (uint32_t)pieces.size();
         uint64_t long_pos = 0;
         for (uint32_t s = first; s < first + n_seg; ++s) {
             const uint32_t len = ptr[s + 1] - ptr[s];
-            if (len > SL_SHORT) long_pos += len;
+            if (len > SL_SHORT) P.all_short = false;
+            if (len > SL_MEDIUM) long_pos += len;
         }
-        P.all_short = long_pos == 0;
         if (P.all_short) {
             P.n_short = n_seg;
-            P.piece_hi = P.piece_lo;
             return P;
         }
-        uint64_t len = (long_pos + target_warps - 1) / std::max<uint32_t>(1, target_warps);
-        len = std::min<uint64_t>(4096, std::max<uint64_t>(512, (len + 127) / 128 * 128));
+        uint64_t len = (long_pos + target_blocks - 1) / std::max<uint32_t>(1, target_blocks);
+        len = std::min<uint64_t>(16384, std::max<uint64_t>(SL_MEDIUM, (len + 127) / 128 * 128));
         for (uint32_t s = first; s < first + n_seg; ++s) {
             const uint32_t a = ptr[s], b = ptr[s + 1];
             if (b - a <= SL_SHORT) {
                 short_ids.push_back(s);
                 ++P.n_short;
+                continue;
+            }
+            if (b - a <= SL_MEDIUM) {
+                medium_ids.push_back(s);
                 continue;
             }
             const uint32_t np = (uint32_t)((b - a + len - 1) / len);
@@ -72,6 +80,7 @@ struct SegBook {
                 pieces.push_back(SLPiece{s, (uint32_t)(a + q * len), (uint32_t)std::min<uint64_t>(b, a + (q + 1) * len),
                                          split});
         }
+        P.medium_hi = (uint32_t)medium_ids.size();
         P.piece_hi = (uint32_t)pieces.size();
         return P;
     }

@@ -39,6 +39,7 @@
 #include "refine.cuh"
 #include "rowsweep.cuh"
 #include "csweep.cuh"
+#include "seglist.cuh"
 #include "tsweep.cuh"
 
 using namespace wgpu;
@@ -180,12 +181,10 @@ struct Tuning {
     uint32_t wide_mean_len = UINT32_MAX;
     bool fuse_rounds = true;     // the small tail of elimination rounds in one block
     bool segthread = true;       // one thread per segment where every segment is short
-    // segmented reductions by warp ranges (segsweep.cuh) instead of block
-    // tiles: 1 = C^T and the adjoint's combines of single-column solves (rows
-    // of ~10-1000 positions, measured faster on the 10M-row panel; at four
-    // columns a lane holds one position and C^T was slower), 2 = every tile
-    // plan at every column count (restrict, means, kept sums, rounds, ...
-    // measured slower), 0 = none
+    // the engine of the segmented reductions: 1 = work lists (seglist.cuh) for
+    // the FP64 plans, warp ranges (segsweep.cuh) for the FP32 C^T and adjoint
+    // combines of one column, block tiles (segreduce.cuh) for the other FP32
+    // plans; 2 = warp ranges for every plan; 0 = block tiles for every plan
     int warp_ranges = 1;
     // cross-tabs of the additive-Schwarz set-up on the GPU (xtab.cu): 1 for
     // designs of at least XTAB_MIN_OBS observations, 2 always, 0 never
@@ -353,6 +352,58 @@ void launch_sr(const F& f, const DevPlan& p, uint32_t lo, uint32_t hi, const int
     ++g_launches;
 }
 
+// The device side of a SegBook (lists, partials, counters), for every K.
+struct DevBook {
+    uint32_t *short_ids = nullptr, *medium_ids = nullptr;
+    SLPiece* pieces = nullptr;
+    SLSplit* splits = nullptr;
+    double* part = nullptr;
+    unsigned* counters = nullptr;
+    void upload(Arena& A, const SegBook& b) {
+        short_ids = A.upload(b.short_ids);
+        medium_ids = A.upload(b.medium_ids);
+        pieces = A.upload(b.pieces);
+        splits = A.upload(b.splits);
+        part = A.alloc<double>(b.splits.empty() ? 1 : b.pieces.size() * 8);   // up to eight columns
+        counters = A.alloc<unsigned>(b.splits.size());
+    }
+};
+
+// pieces a problem's long segments are cut into: one wave of resident blocks
+constexpr uint32_t SL_TARGET_BLOCKS = 148 * 6;
+
+template <class F, int K>
+void launch_sl(const F& f, const DevBook& b, const SLPart& p, const uint32_t* ptr, const int* skip, cudaStream_t st) {
+    if constexpr (K == 1 && F::STAGED) {
+        if (p.all_short) {
+            if (!p.n_short) return;
+            launch_k(k_segstage<F>, (p.n_short + SL_THREADS - 1) / SL_THREADS, SL_THREADS, 0, st, f, ptr, p.first,
+                     p.n_short, skip);
+            ++g_launches;
+            return;
+        }
+    }
+    SLDev L;
+    L.ptr = ptr;
+    L.short_ids = p.all_short ? nullptr : b.short_ids + p.short_off;
+    L.medium_ids = b.medium_ids + p.medium_lo;
+    L.first = p.first;
+    L.n_short = p.n_short;
+    L.n_medium = p.medium_hi - p.medium_lo;
+    L.n_piece = p.piece_hi - p.piece_lo;
+    L.medium_blocks = (L.n_medium + SL_WARPS - 1) / SL_WARPS;
+    L.pieces = b.pieces + p.piece_lo;
+    L.piece_lo = p.piece_lo;
+    L.splits = b.splits;
+    L.part = b.part;
+    L.counters = b.counters;
+    const uint32_t short_blocks = (uint32_t)(((uint64_t)p.n_short * fl_per_row<K>() + SL_THREADS - 1) / SL_THREADS);
+    const uint32_t grid = L.n_piece + L.medium_blocks + short_blocks;
+    if (!grid) return;
+    launch_k(k_seglist<F, K>, grid, SL_THREADS, 0, st, f, L, skip);
+    ++g_launches;
+}
+
 int k_bucket(uint64_t k) { return k <= 1 ? 1 : k <= 2 ? 2 : k <= 4 ? 4 : 8; }
 
 // MlsmrOptions extras of one solve (lsmr.rs:155-171): warm start (device,
@@ -392,6 +443,9 @@ struct within_preconditioner {
     SegProb *p_restrict = nullptr, *p_ct = nullptr, *p_kept = nullptr, *p_dense = nullptr,
             *p_fwd = nullptr, *p_bwd = nullptr, *p_c = nullptr, *p_prolong = nullptr,
             *p_core = nullptr;
+    // the same steps' segment pointers
+    const uint32_t *ct_ptr = nullptr, *dense_ptr = nullptr, *fwd_ptr = nullptr, *bwd_ptr = nullptr, *c_ptr = nullptr,
+                   *dof_ptr = nullptr, *core_ptr = nullptr;
     bool has_dense = false, has_core = false;
     uint32_t n_rounds = 0;
     std::mutex mu;
@@ -470,6 +524,13 @@ void upload_schwarz_image(within_preconditioner& P) {
     P.p_c = one(c_ptr);
     P.p_prolong = one(dof_ptr);
     P.p_core = one(core_ptr);
+    P.ct_ptr = ct_ptr;
+    P.dense_ptr = dense_ptr;
+    P.fwd_ptr = fwd_ptr;
+    P.bwd_ptr = bwd_ptr;
+    P.c_ptr = c_ptr;
+    P.dof_ptr = dof_ptr;
+    P.core_ptr = core_ptr;
     P.has_dense = H.dense_rows_ptr.size() > 1;
     P.has_core = H.core_rows_ptr.size() > 1;
     P.n_rounds = H.n_rounds;
@@ -567,6 +628,7 @@ struct KPlans {
     SchwarzWork w;
     SchwarzWorkT<float> wf;   // mixed-precision inner solve, allocated on first use
     bool ready = false;
+    bool plans = false;       // the tile / range plans and one-thread round tables are built
 };
 
 }  // namespace
@@ -575,15 +637,59 @@ struct SchwarzUser {
     Arena arena;
     KPlans kp[4];
     Tuning tuning;
+    // the list engine's lists (FP64 applies), shared by every column bucket
+    struct Lists {
+        bool ready = false;
+        DevBook book;
+        SLPart restrict_, ct, kept, dense, core, c, prolong;
+        std::vector<SLPart> fwd, bwd;
+    } lists;
 };
 
 within_preconditioner::~within_preconditioner() { delete standalone; }
 
 namespace {
 
-KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K) {
+// Whether the FP64 plans of this tuning run on the list engine: the default
+// record (on the 10M-row panel an iteration's segmented sums take 190 us on
+// lists and 280 us on tiles and ranges, at eight columns 620 and 1270 us).  The
+// knobs of the other engines -- tiles or ranges, wide tiles, no one-thread
+// segments, C by groups of lanes -- select those.  The FP32 applies always do:
+// an FP32 sum in another order rounds differently, and the mixed solve's x is
+// pinned to those roundings in the directions the design does not determine.
+bool use_lists(const Tuning& t) {
+    return t.warp_ranges == 1 && t.segthread && !t.vector_rows && t.wide_mean_len == UINT32_MAX;
+}
+
+void ensure_lists(SchwarzUser& U, const within_preconditioner& P) {
+    auto& L = U.lists;
+    if (L.ready) return;
+    const SchwarzHost& H = P.host;
+    SegBook b;
+    auto whole = [&](const std::vector<uint32_t>& ptr) {
+        return b.add(ptr.data(), 0, ptr.empty() ? 0 : (uint32_t)ptr.size() - 1, SL_TARGET_BLOCKS);
+    };
+    L.restrict_ = whole(H.loc_ptr);
+    L.ct = whole(H.ct_ptr);
+    L.kept = whole(H.kept_ptr);
+    L.dense = whole(H.dense_rows_ptr);
+    L.core = whole(H.core_rows_ptr);
+    L.c = whole(H.c_ptr);
+    L.prolong = whole(H.dof_ptr);
+    for (uint32_t r = 0; r < H.n_rounds; ++r) {
+        L.fwd.push_back(b.add(H.fwd_ptr.data(), H.fwd_round_ptr[r], H.fwd_round_ptr[r + 1] - H.fwd_round_ptr[r],
+                              SL_TARGET_BLOCKS));
+        L.bwd.push_back(b.add(H.bwd_ptr.data(), H.bwd_round_ptr[r], H.bwd_round_ptr[r + 1] - H.bwd_round_ptr[r],
+                              SL_TARGET_BLOCKS));
+    }
+    L.book.upload(U.arena, b);
+    L.ready = true;
+}
+
+// The tile and warp-range plans of one column bucket and its round tables.
+void ensure_tile_plans(SchwarzUser& U, const within_preconditioner& P, int K) {
     KPlans& kp = U.kp[kidx(K)];
-    if (kp.ready) return kp;
+    if (kp.plans) return;
     const SchwarzHost& H = P.host;
     Arena& A = U.arena;
     const int T = plan_tile(K, false);
@@ -662,6 +768,19 @@ KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K
     };
     kp.fwd_thread = round_thread(H.fwd_round_ptr, H.fwd_ptr);
     kp.bwd_thread = round_thread(H.bwd_round_ptr, H.bwd_ptr);
+    kp.plans = true;
+}
+
+// The rounds that run as one single-block launch per direction.
+void ensure_fused_rounds(SchwarzUser& U, const within_preconditioner& P, int K) {
+    KPlans& kp = U.kp[kidx(K)];
+    const SchwarzHost& H = P.host;
+    Arena& A = U.arena;
+    const bool segt_on = U.tuning.segthread;
+    auto short_round = [&](const std::vector<uint32_t>& rptr, const std::vector<uint32_t>& ptr, uint32_t r) {
+        const uint32_t m = rptr[r + 1] - rptr[r];
+        return m == 0 || seg_max_len(ptr.data() + rptr[r], m) <= SEGT_MAX_LEN;
+    };
     // the fused tail: the longest suffix of rounds that are one-thread rounds
     // in both directions with at most RF_MAX_ROWS rows (WITHIN_FUSE_ROUNDS=0: none)
     {
@@ -671,8 +790,8 @@ KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K
         auto ok = [&](uint32_t r) {
             const uint32_t fr = H.fwd_round_ptr[r + 1] - H.fwd_round_ptr[r];
             const uint32_t br = H.bwd_round_ptr[r + 1] - H.bwd_round_ptr[r];
-            return (fr == 0 || kp.fwd_thread[r]) && (br == 0 || kp.bwd_thread[r]) && fr <= RF_MAX_ROWS &&
-                   br <= RF_MAX_ROWS;
+            return fr <= RF_MAX_ROWS && br <= RF_MAX_ROWS && short_round(H.fwd_round_ptr, H.fwd_ptr, r) &&
+                   short_round(H.bwd_round_ptr, H.bwd_ptr, r);
         };
         while (fuse_on && lo > 0 && ok(lo - 1)) --lo;
         if (nr - lo >= 2) {
@@ -687,6 +806,16 @@ KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K
             kp.bwd_rows = A.upload(br);
         }
     }
+}
+
+KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K) {
+    KPlans& kp = U.kp[kidx(K)];
+    if (kp.ready) return kp;
+    const SchwarzHost& H = P.host;
+    Arena& A = U.arena;
+    if (use_lists(U.tuning)) ensure_lists(U, P);
+    else ensure_tile_plans(U, P, K);
+    ensure_fused_rounds(U, P, K);
     size_t nl = H.glob.size(), nr = H.n_red, ns = H.n_sub;
     kp.w.rl = A.alloc<double>(nl * K);
     kp.w.sl = A.alloc<double>(nl * K);
@@ -703,6 +832,7 @@ KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K
 // FP32 work vectors of one user (allocated outside any stream capture).
 SchwarzWorkT<float>& schwarz_user_work_f(SchwarzUser& U, const within_preconditioner& P, int K) {
     KPlans& kp = schwarz_user_plans(U, P, K);
+    ensure_tile_plans(U, P, K);
     if (!kp.wf.rl) {
         const SchwarzHost& H = P.host;
         size_t nl = H.glob.size(), nr = H.n_red, ns = H.n_sub;
@@ -739,13 +869,44 @@ void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, c
     S.m1 = w->m1;
     S.m2 = w->m2;
     S.m3 = w->m3;
+    const bool fused = kp.fuse_hi > kp.fuse_lo;
+    const uint32_t r_fwd_end = fused ? kp.fuse_lo : P.n_rounds;
+    using FF = FwdF<K, T>;
+    using BF = BwdF<K, T>;
+    auto fused_rounds = [&](bool backward) {
+        if (!fused) return;
+        if (backward)
+            launch_k(rounds_fused_kernel<BF, K>, 1, RF_THREADS, 0, st, BF{P.p_bwd, S}, kp.bwd_rows, kp.fuse_lo,
+                     kp.fuse_hi, 1, skip);
+        else
+            launch_k(rounds_fused_kernel<FF, K>, 1, RF_THREADS, 0, st, FF{P.p_fwd, S}, kp.fwd_rows, kp.fuse_lo,
+                     kp.fuse_hi, 0, skip);
+        ++g_launches;
+    };
+    if constexpr (sizeof(T) == 8) {
+        if (use_lists(U.tuning)) {
+            const auto& L = U.lists;
+            const DevBook& b = L.book;
+            launch_sl<SlRestrict<K>, K>({{S}, r}, b, L.restrict_, S.loc_ptr, skip, st);
+            launch_sl<SlCt<K>, K>({{S}}, b, L.ct, P.ct_ptr, skip, st);
+            launch_sl<SlKeptSum<K>, K>({{S}}, b, L.kept, S.kept_ptr, skip, st);
+            if (P.has_dense) launch_sl<SlDense<K>, K>({{S}}, b, L.dense, P.dense_ptr, skip, st);
+            for (uint32_t q = 0; q < r_fwd_end; ++q) launch_sl<SlFwd<K>, K>({{S}}, b, L.fwd[q], P.fwd_ptr, skip, st);
+            fused_rounds(false);
+            if (P.has_core) launch_sl<SlCore<K>, K>({{S}}, b, L.core, P.core_ptr, skip, st);
+            fused_rounds(true);
+            for (uint32_t q = r_fwd_end; q-- > 0;) launch_sl<SlBwd<K>, K>({{S}}, b, L.bwd[q], P.bwd_ptr, skip, st);
+            launch_sl<SlC<K>, K>({{S}}, b, L.c, P.c_ptr, skip, st);
+            launch_sl<SlMean<K>, K>({{S}}, b, L.restrict_, S.loc_ptr, skip, st);
+            launch_sl<SlProlong<K>, K>({{S}, z}, b, L.prolong, P.dof_ptr, skip, st);
+            return;
+        }
+    }
     using RF = RestrictF<K, T>;
     using CtFT = CtF<K, T>;
     using KS = KeptSumF<K, T>;
     using DF = DenseF<K, T>;
-    using FF = FwdF<K, T>;
     using CoF = CoreF<K, T>;
-    using BF = BwdF<K, T>;
     using CFT = CF<K, T>;
     using MF = MeanF<K, T>;
     using PF = ProlongF<K, T>;
@@ -753,23 +914,13 @@ void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, c
     launch_sr<CtFT, K>(CtFT{P.p_ct, S}, kp.ct, 0, kp.ct.n_tiles, skip, st);
     launch_sr<KS, K>(KS{P.p_kept, S}, kp.kept, 0, kp.kept.n_tiles, skip, st);
     if (P.has_dense) launch_sr<DF, K>(DF{P.p_dense, S}, kp.dense, 0, kp.dense.n_tiles, skip, st);
-    const bool fused = kp.fuse_hi > kp.fuse_lo;
-    const uint32_t r_fwd_end = fused ? kp.fuse_lo : P.n_rounds;
     for (uint32_t r = 0; r < r_fwd_end; ++r) {
         if (kp.fwd_thread[r]) launch_segthread<FF, K>(FF{P.p_fwd, S}, r, kp.fwd_thread[r], skip, st);
         else launch_sr<FF, K>(FF{P.p_fwd, S}, kp.fwd, kp.fwd.range_lo[r], kp.fwd.range_hi[r], skip, st);
     }
-    if (fused) {
-        launch_k(rounds_fused_kernel<FF, K>, 1, RF_THREADS, 0, st, FF{P.p_fwd, S}, kp.fwd_rows, kp.fuse_lo, kp.fuse_hi, 0,
-                                                              skip);
-        ++g_launches;
-    }
+    fused_rounds(false);
     if (P.has_core) launch_sr<CoF, K>(CoF{P.p_core, S}, kp.core, 0, kp.core.n_tiles, skip, st);
-    if (fused) {
-        launch_k(rounds_fused_kernel<BF, K>, 1, RF_THREADS, 0, st, BF{P.p_bwd, S}, kp.bwd_rows, kp.fuse_lo, kp.fuse_hi, 1,
-                                                              skip);
-        ++g_launches;
-    }
+    fused_rounds(true);
     for (uint32_t r = r_fwd_end; r-- > 0;) {
         if (kp.bwd_thread[r]) launch_segthread<BF, K>(BF{P.p_bwd, S}, r, kp.bwd_thread[r], skip, st);
         else launch_sr<BF, K>(BF{P.p_bwd, S}, kp.bwd, kp.bwd.range_lo[r], kp.bwd.range_hi[r], skip, st);
@@ -853,7 +1004,10 @@ struct within_solver {
         size_t smem = 0;
         std::vector<ScatterProb> rest_host;   // run combines + full-resolution rest terms
         std::vector<std::vector<uint32_t>> rest_ptrs;
-        DevPlan rest;
+        DevPlan rest;                        // tile / range plan (FP32, or the list engine off)
+        bool rest_plan = false;
+        DevBook rest_book;                   // list-engine lists (FP64)
+        std::vector<SLPart> rest_parts;      // one per problem
         ScatterProb* rest_probs = nullptr;
         ScatterProb* rest_probs_f = nullptr;
         uint32_t n_rest = 0;
@@ -1092,6 +1246,35 @@ bool launch_tgather(within_solver& s, const double* x, const double* yint, doubl
     return true;
 }
 
+// The tile or warp-range plan of the adjoint's rest.
+template <int K>
+void ensure_rest_plan(within_solver& s, within_solver::RowSweepK& rk) {
+    if (rk.rest_plan || !rk.n_rest) return;
+    Arena& A = s.arena;
+    uint64_t pos = 0, segs = 0;
+    for (const auto& lp : rk.rest_ptrs) {
+        pos += lp.back() - lp.front();
+        segs += lp.size() - 1;
+    }
+    if (s.schwarz.tuning.warp_ranges >= 2 || (s.schwarz.tuning.warp_ranges == 1 && K == 1)) {
+        SSHostPlan sp;
+        const uint32_t L = ss_range_len(pos, ss_target_warps(K));
+        for (size_t i = 0; i < rk.rest_host.size(); ++i)
+            sp.add((uint32_t)i, rk.rest_ptrs[i].data(), (uint32_t)rk.rest_ptrs[i].size() - 1, L);
+        rk.rest = make_ss_plan(A, sp, K);
+    } else {
+        const bool wide = plan_wide(K, pos, segs, s.schwarz.tuning.wide_mean_len);
+        const int Ttile = plan_tile(K, wide);
+        HostPlan hp;
+        for (size_t i = 0; i < rk.rest_host.size(); ++i)
+            hp.add((uint32_t)i, rk.rest_ptrs[i].data(), (uint32_t)rk.rest_ptrs[i].size() - 1, Ttile);
+        rk.rest = make_plan(A, hp, K);
+        rk.rest.wide = wide;
+    }
+    rk.rest_probs = A.upload(rk.rest_host);
+    rk.rest_plan = true;
+}
+
 // Classifies the terms for the warp-range row sweep and builds its tables
 // (rowsweep.cuh): range bases of the run ordinals, the crossing-run fix-ups,
 // the level-sorted run combines and the remaining full-resolution terms.
@@ -1291,27 +1474,14 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
     if (!share) rk.atu = A.alloc<double>(s.n_dofs * K);
     rk.n_rest = (uint32_t)rk.rest_host.size();
     if (rk.n_rest) {
-        uint64_t pos = 0, segs = 0;
-        for (const auto& lp : rk.rest_ptrs) {
-            pos += lp.back() - lp.front();
-            segs += lp.size() - 1;
-        }
-        if (s.schwarz.tuning.warp_ranges >= 2 || (s.schwarz.tuning.warp_ranges == 1 && K == 1)) {
-            SSHostPlan sp;
-            const uint32_t L = ss_range_len(pos, ss_target_warps(K));
-            for (size_t i = 0; i < rk.rest_host.size(); ++i)
-                sp.add((uint32_t)i, rk.rest_ptrs[i].data(), (uint32_t)rk.rest_ptrs[i].size() - 1, L);
-            rk.rest = make_ss_plan(A, sp, K);
+        if (use_lists(s.schwarz.tuning)) {
+            SegBook book;
+            for (const auto& lp : rk.rest_ptrs)
+                rk.rest_parts.push_back(book.add(lp.data(), 0, (uint32_t)lp.size() - 1, SL_TARGET_BLOCKS));
+            rk.rest_book.upload(A, book);
         } else {
-            const bool wide = plan_wide(K, pos, segs, s.schwarz.tuning.wide_mean_len);
-            const int Ttile = plan_tile(K, wide);
-            HostPlan hp;
-            for (size_t i = 0; i < rk.rest_host.size(); ++i)
-                hp.add((uint32_t)i, rk.rest_ptrs[i].data(), (uint32_t)rk.rest_ptrs[i].size() - 1, Ttile);
-            rk.rest = make_plan(A, hp, K);
-            rk.rest.wide = wide;
+            ensure_rest_plan<K>(s, rk);
         }
-        rk.rest_probs = A.upload(rk.rest_host);
     }
     // dynamic shared memory above the default needs the opt-in (set outside any capture)
     // The dynamic shared-memory ceiling is a property of the kernel function
@@ -1376,6 +1546,7 @@ void ensure_rowsweep_f(within_solver& s) {
     auto& rk = ensure_rowsweep<K>(s);
     if (rk.cs && !s.rsw_f[kidx(K)].ready) build_rowsweep<K>(s, s.rsw_f[kidx(K)], &rk);
     if (rk.rest_probs_f || !rk.n_rest) return;
+    ensure_rest_plan<K>(s, rk);
     std::vector<ScatterProb> pf = rk.rest_host;
     for (auto& pr : pf) {
         pr.load_f = nullptr;
@@ -1447,6 +1618,12 @@ void rowsweep_rest(within_solver& s, within_solver::RowSweepK& rk, const T* u, T
                    cudaStream_t st) {
     if (!rk.n_rest) return;
     if constexpr (sizeof(T) == 8) {
+        if (!rk.rest_parts.empty()) {
+            for (size_t i = 0; i < rk.rest_parts.size(); ++i)
+                launch_sl<SlScatter<K>, K>({rk.rest_host[i], u, s.op.sqrt_w, out}, rk.rest_book, rk.rest_parts[i],
+                                           rk.rest_host[i].seg_ptr, skip, st);
+            return;
+        }
         ScatterF<K, 0> f{rk.rest_probs, u, s.op.sqrt_w, out, nullptr};
         launch_sr<ScatterF<K, 0>, K>(f, rk.rest, 0, rk.rest.n_tiles, skip, st);
     } else {
