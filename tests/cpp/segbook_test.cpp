@@ -1,5 +1,7 @@
 // SegBook: every position of every problem lies in exactly one short segment,
 // medium segment or piece; pieces of a split segment are consecutive.
+// NarrowRounds: every row once, its entries in its lanes, aligned passes.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <random>
@@ -58,6 +60,54 @@ int main() {
         }
         for (uint32_t s = 0; s < n; ++s) CHECK(segs[s] == (s >= first ? 1 : 0));
         for (uint32_t q = 0; q < ptr.back(); ++q) CHECK(seen[q] == (q >= ptr[first] ? 1 : 0));
+    }
+    const uint32_t lens[] = {0, 1, RP_LANES, RP_LANES + 1, 17, 45, RP_ENTRIES / 32 * RP_LANES};
+    for (int trial = 0; trial < 40; ++trial) {
+        const uint32_t n = trial < 3 ? trial : 1 + rng() % 700, zero = 100000;
+        std::vector<uint32_t> ptr(1, rng() % 5), col, id;
+        std::vector<double> val;
+        for (uint32_t r = 0; r < n; ++r) {
+            ptr.push_back(ptr.back() + lens[rng() % (trial % 4 == 0 ? 7 : 6)]);
+            id.push_back(5000 + r);
+        }
+        for (uint32_t e = 0; e < ptr.back(); ++e) {
+            col.push_back(rng() % 5000);
+            val.push_back(1.0 + e);
+        }
+        NarrowRounds N;
+        const uint32_t cut = n ? rng() % (n + 1) : 0;   // two rounds
+        CHECK(N.add(ptr.data(), col.data(), val.data(), id.data(), 0, cut, zero));
+        const size_t first_pass2 = N.pass.size();
+        CHECK(N.add(ptr.data(), col.data(), val.data(), id.data(), cut, n, zero));
+        CHECK(N.val.size() == N.col.size() && N.row.size() == N.slice.size() * RP_SLICE);
+        std::vector<double> sum(n, 0.0), want(n, 0.0);
+        std::vector<int> seen(n, 0);
+        for (uint32_t r = 0; r < n; ++r)
+            for (uint32_t e = ptr[r]; e < ptr[r + 1]; ++e) want[r] += val[e] * (1.0 + col[e]);
+        for (size_t p = 0; p < N.pass.size(); ++p) {
+            const RPass& P = N.pass[p];
+            CHECK(P.n_slice >= 1 && P.n_slice <= RP_WARPS && P.n_ent <= RP_ENTRIES && P.n_ent % 32 == 0);
+            CHECK(P.e0 % 32 == 0 && P.s0 % 2 == 0 && P.s0 + P.n_slice <= N.slice.size());
+            for (uint32_t q = 0; q < P.n_slice; ++q) {
+                const RSlice& sl = N.slice[P.s0 + q];
+                CHECK(sl.first + sl.width * 32 <= P.n_ent);
+                for (uint32_t l = 0; l < 32; ++l) {
+                    const uint32_t row = N.row[(P.s0 + q) * RP_SLICE + l / RP_LANES];
+                    if (row != zero && l % RP_LANES == 0) {
+                        ++seen[row - 5000];
+                        CHECK((row - 5000 < cut) == (p < first_pass2));
+                    }
+                    for (uint32_t j = 0; j < sl.width; ++j) {
+                        const size_t at = (size_t)P.e0 + sl.first + j * 32 + l;
+                        if (N.col[at] == zero) CHECK(N.val[at] == 0.0);
+                        else sum[row - 5000] += N.val[at] * (1.0 + N.col[at]);
+                    }
+                }
+            }
+        }
+        for (uint32_t r = 0; r < n; ++r) CHECK(seen[r] == 1 && std::abs(sum[r] - want[r]) <= 1e-12 * want[r]);
+        std::vector<uint32_t> wide = {0, RP_ENTRIES / 32 * RP_LANES + 1};
+        CHECK(!N.add(wide.data(), col.data(), val.data(), id.data(), 0, 1, zero));
     }
     std::printf("ok\n");
     return 0;

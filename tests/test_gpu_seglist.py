@@ -19,12 +19,18 @@ def design(kind, rng):
         g = np.repeat(np.arange(6_000), 4)
         return np.asfortranarray(np.column_stack([2 * g + rng.integers(0, 2, g.size),
                                                   2 * g + rng.integers(0, 2, g.size)]).astype(np.uint32))
+    if kind == "rounds":     # a deep factor: 30 and more narrow elimination rounds and a dense core
+        from within_b200 import workloads as WL
+        return WL.fixest_like(n=600_000)[0]
+    if kind == "rounds_wide":   # a factor whose first rounds are launches of their own
+        return np.asfortranarray(np.column_stack([rng.integers(0, 30_000, 150_000), rng.integers(0, 6_000, 150_000)])
+                                 .astype(np.uint32))
     # unused levels: empty segments of the prolongation and of the adjoint's rest
     a, b = 3 * rng.integers(0, 700, 40_000), 2 * rng.integers(0, 900, 40_000)
     return np.asfortranarray(np.column_stack([a, b, rng.integers(0, 4, 40_000)]).astype(np.uint32))
 
 
-@pytest.mark.parametrize("kind", ["panel", "islands", "gaps"])
+@pytest.mark.parametrize("kind", ["panel", "islands", "gaps", "rounds", "rounds_wide"])
 @pytest.mark.parametrize("k", [1, 2, 3, 8])
 def test_lists_match_tiles(wb, kind, k):
     rng = np.random.default_rng(11 + k)

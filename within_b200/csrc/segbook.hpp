@@ -86,4 +86,66 @@ struct SegBook {
     }
 };
 
+// Slices of the narrow rounds of a triangular solve (k_rounds, seglist.cuh).
+constexpr uint32_t RP_THREADS = 992, RP_WARPS = RP_THREADS / 32;
+constexpr uint32_t RP_LANES = 4;              // lanes per row
+constexpr uint32_t RP_SLICE = 32 / RP_LANES;  // rows per warp
+constexpr uint32_t RP_ENTRIES = 4096;         // most entries of one pass (padding counted)
+constexpr uint32_t RP_STAGES = 3;
+
+struct RPass {
+    uint32_t e0, n_ent;       // entries [e0, e0 + n_ent) of val / col
+    uint32_t s0, n_slice;     // slices [s0, s0 + n_slice); slice lists start at even s0
+};
+struct RSlice {
+    uint32_t first, width;    // first entry relative to the pass, entries per lane
+};
+
+struct NarrowRounds {
+    std::vector<double> val;
+    std::vector<uint32_t> col, row;
+    std::vector<RSlice> slice;
+    std::vector<RPass> pass;
+
+    // Appends one round: rows [lo, hi) of the factor (ptr, col, val in CSR, id[r]
+    // the reduced slot of row r).  Padding entries and rows name slot `zero`.
+    // false (nothing appended): a row alone is wider than a pass.
+    bool add(const uint32_t* ptr, const uint32_t* c, const double* v, const uint32_t* id, uint32_t lo, uint32_t hi,
+             uint32_t zero) {
+        std::vector<uint32_t> order(hi - lo);
+        for (uint32_t i = 0; i < hi - lo; ++i) order[i] = lo + i;
+        auto len = [&](uint32_t r) { return ptr[r + 1] - ptr[r]; };
+        std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return len(a) > len(b); });
+        if (!order.empty() && (len(order[0]) + RP_LANES - 1) / RP_LANES * 32 > RP_ENTRIES) return false;
+        for (uint32_t i = 0; i < order.size();) {
+            RPass P{(uint32_t)val.size(), 0, (uint32_t)slice.size(), 0};
+            while (i < order.size() && P.n_slice < RP_WARPS) {
+                const uint32_t w = (len(order[i]) + RP_LANES - 1) / RP_LANES;   // the slice's longest row
+                if (P.n_ent + w * 32 > RP_ENTRIES) break;
+                slice.push_back(RSlice{P.n_ent, w});
+                val.resize(val.size() + (size_t)w * 32, 0.0);
+                col.resize(col.size() + (size_t)w * 32, zero);
+                for (uint32_t q = 0; q < RP_SLICE; ++q) {
+                    const bool on = i + q < order.size();
+                    row.push_back(on ? id[order[i + q]] : zero);
+                    for (uint32_t e = 0; on && e < len(order[i + q]); ++e) {
+                        const size_t at = (size_t)P.e0 + P.n_ent + (e / RP_LANES) * 32 + q * RP_LANES + e % RP_LANES;
+                        val[at] = v[ptr[order[i + q]] + e];
+                        col[at] = c[ptr[order[i + q]] + e];
+                    }
+                }
+                P.n_ent += w * 32;
+                ++P.n_slice;
+                i += RP_SLICE;
+            }
+            if (slice.size() % 2) {   // the next pass's slices start 16-byte aligned
+                slice.push_back(RSlice{0, 0});
+                row.insert(row.end(), RP_SLICE, zero);
+            }
+            pass.push_back(P);
+        }
+        return true;
+    }
+};
+
 }  // namespace wgpu

@@ -31,6 +31,7 @@
 #include "pdl.cuh"
 #include <cstdint>
 
+#include "bulk.cuh"
 #include "kernels.cuh"
 #include "segbook.hpp"
 
@@ -505,6 +506,179 @@ struct SlProlong : SlBase<K> {
     __device__ void emit(uint32_t dof, int c0, const Pre&, const V& s) const { B::st(z, dof, c0, s); }
 };
 #undef SL_TYPES
+
+// ---------------------------------------------------------------------------
+// The narrow rounds of the factor's triangular solves in one launch per
+// direction: one block per column keeps that column's reduced vector in shared
+// memory and walks the rounds, one block barrier per pass.  A round of a few
+// hundred rows of ten entries is 2 us of latency (index, operand, emit, each
+// from L2) and 2 us of launch for 20 ns of traffic; here the entries are copied
+// into shared memory RP_STAGES - 1 passes ahead, right-hand sides are formed
+// before the first pass and results written after the last, so a pass touches
+// shared memory only.  What bounds it then is the one SM's issue rate, so the
+// host packs the rows into slices (NarrowRounds, segbook.hpp): the rows of a
+// round sorted by length, RP_SLICE rows per warp, RP_LANES lanes per row, padded
+// to the slice's longest row -- no row pointers, no bounds, conflict-free reads
+// of index and value.  33 rounds of a factor of 4,368 vertices and 47,000 entries
+// (1,000,000-row design with a 4,348-level factor), per direction: 200 us as
+// launches, 40 us forward and 32 us backward here (0.9 us per pass: barrier,
+// index, operand, sum and write-back in sequence).  Reading the rows' entries
+// from L2 one pass ahead took 56 us, copying them with every thread 50 us.
+struct RStage {
+    double val[RP_ENTRIES];
+    uint32_t col[RP_ENTRIES];
+    uint32_t row[RP_WARPS * RP_SLICE];
+    uint2 slice[RP_WARPS + RP_WARPS % 2];   // copied in pairs
+};
+static_assert(sizeof(RStage) % 16 == 0 && RP_WARPS * 32 == RP_THREADS, "16-byte aligned stages, one slice per warp");
+
+// device arrays of a NarrowRounds
+struct RDev {
+    const double* val;
+    const uint32_t *col, *row;
+    const uint2* slice;
+    const RPass* pass;
+    uint32_t n_pass;
+};
+
+// BACKWARD false: y_u = b_u - sum L[u, v] y_v and z_u = y_u / d_u for the factor
+// rows [row_lo, row_hi) (the y of earlier rows from memory);
+// true: x_v = z_v - sum L[u, v] x_u.
+template <int K, bool BACKWARD>
+__global__ void __launch_bounds__(RP_THREADS + 32)
+k_rounds(SchwarzDev S, RDev R, uint32_t row_lo, uint32_t row_hi, uint32_t n_red, int* err,
+         const int* __restrict__ skip) {
+    pdl_wait();
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) unsigned char rp_smem[];
+    if (skip && *skip) return;
+    const int k = blockIdx.x;   // this block's column
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t tid = threadIdx.x, wid = tid >> 5, lane = tid & 31u;
+    const uint32_t* __restrict__ rows = BACKWARD ? S.bwd_row : S.fwd_row;
+    RStage* stage = reinterpret_cast<RStage*>(rp_smem);
+    RPass* pass = reinterpret_cast<RPass*>(rp_smem + RP_STAGES * sizeof(RStage));
+    double* vec = reinterpret_cast<double*>(pass + R.n_pass);   // n_red values and a zero for the padding
+    __shared__ __align__(8) uint64_t bar[RP_STAGES];
+    for (uint32_t i = tid; i < R.n_pass; i += RP_THREADS + 32) pass[i] = R.pass[i];
+    if (tid == 0) {
+        for (uint32_t i = 0; i < RP_STAGES; ++i) mbar_init(&bar[i], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    // the last warp's first lane has the passes copied (sizes are multiples of 16 bytes), the others sum
+    const bool copies = tid == RP_THREADS;
+    auto issue = [&](uint32_t p) {
+        if (p >= R.n_pass) return;
+        const RPass q = pass[p];
+        RStage& G = stage[p % RP_STAGES];
+        uint64_t* bp = &bar[p % RP_STAGES];
+        const uint32_t sb = (q.n_slice + 1) / 2 * 16, rb = q.n_slice * RP_SLICE * 4;
+        mbar_arrive_expect_tx(bp, q.n_ent * 12 + sb + rb);
+        if (q.n_ent) {
+            bulk_g2s(G.val, R.val + q.e0, q.n_ent * 8, bp);
+            bulk_g2s(G.col, R.col + q.e0, q.n_ent * 4, bp);
+        }
+        bulk_g2s(G.row, R.row + q.s0 * RP_SLICE, rb, bp);
+        bulk_g2s(G.slice, R.slice + q.s0, sb, bp);
+    };
+    if (copies)
+        for (uint32_t i = 0; i + 1 < RP_STAGES; ++i) issue(i);
+    // the column's values, eight per thread in flight
+    for (uint32_t u0 = tid; wid < RP_WARPS && u0 < n_red; u0 += 8 * RP_THREADS) {
+        double x[8];
+        uint32_t sub[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t u = min(u0 + j * RP_THREADS, n_red - 1);
+            x[j] = (BACKWARD ? S.xv : S.rb)[(size_t)u * K + k];
+            sub[j] = BACKWARD ? 0u : __ldg(S.red_sub + u);
+        }
+        if constexpr (!BACKWARD) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] -= S.m2[(size_t)sub[j] * K + k];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (u0 + j * RP_THREADS < n_red) vec[u0 + j * RP_THREADS] = x[j];
+    }
+    if (tid == 0) vec[n_red] = 0.0;
+    if (!BACKWARD && row_lo > 0) {   // rounds that ran as launches of their own
+        __syncthreads();
+        for (uint32_t r = tid; wid < RP_WARPS && r < row_lo; r += RP_THREADS) {
+            const uint32_t u = __ldg(rows + r);
+            vec[u] = S.yv[(size_t)u * K + k];
+        }
+    }
+    bool failed = false;
+    uint32_t p = 0;
+    for (; p < R.n_pass; ++p) {
+        const bool landed = mbar_wait_bounded(&bar[p % RP_STAGES], (p / RP_STAGES) & 1u);
+        // pass p's copies and the previous pass's sums are visible to every thread
+        if (__syncthreads_or(!landed)) {
+            failed = true;
+            break;
+        }
+        if (copies) {   // into the stage of pass p - 1, which every warp has left
+            fence_proxy_async_smem();
+            issue(p + RP_STAGES - 1);
+        }
+        if (wid == RP_WARPS) continue;
+        if (wid >= pass[p].n_slice) continue;   // whole warps
+        const RStage& G = stage[p % RP_STAGES];
+        const uint2 sl = G.slice[wid];   // first entry in the pass, entries per lane
+        const uint32_t row = G.row[wid * RP_SLICE + lane / RP_LANES];   // padding rows: the zero
+        const double* gv = G.val + sl.x + lane;
+        const uint32_t* gc = G.col + sl.x + lane;
+        double s = 0.0;
+        for (uint32_t j0 = 0; j0 < sl.y; j0 += 4) {
+            double v[4], x[4];
+            uint32_t c[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {   // past the width: the last entry again, not added
+                const uint32_t i = min(j0 + j, sl.y - 1) * 32;
+                c[j] = gc[i];
+                v[j] = gv[i];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) x[j] = vec[c[j]];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s += j0 + j < sl.y ? v[j] * x[j] : 0.0;
+        }
+#pragma unroll
+        for (int o = 1; o < (int)RP_LANES; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
+        if (lane % RP_LANES == 0) vec[row] -= s;
+    }
+    if (failed) {   // record it, then wait (bounded) for the copies still in flight
+        if (tid == 0) atomicExch(err, ERR_WAIT_TIMEOUT);
+        for (uint32_t q = p; q < R.n_pass && q + 1 < p + RP_STAGES; ++q)
+            (void)mbar_wait_bounded(&bar[q % RP_STAGES], (q / RP_STAGES) & 1u);
+        return;
+    }
+    __syncthreads();
+    if (wid == RP_WARPS) return;
+    for (uint32_t r0 = row_lo + tid; r0 < row_hi; r0 += 8 * RP_THREADS) {
+        uint32_t u[8];
+        double di[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u[j] = __ldg(rows + min(r0 + j * RP_THREADS, row_hi - 1));
+        if constexpr (!BACKWARD) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) di[j] = __ldg(S.dinv + u[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (r0 + j * RP_THREADS >= row_hi) continue;
+            const double y = vec[u[j]];
+            if constexpr (BACKWARD) {
+                S.xv[(size_t)u[j] * K + k] = y;
+            } else {
+                S.yv[(size_t)u[j] * K + k] = y;
+                S.xv[(size_t)u[j] * K + k] = y * di[j];
+            }
+        }
+    }
+}
 
 // one (term, column) problem of A^T u: run sums by run ordinal, or the rows
 // of the term's level-sorted order

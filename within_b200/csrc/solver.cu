@@ -637,12 +637,18 @@ struct SchwarzUser {
     Arena arena;
     KPlans kp[4];
     Tuning tuning;
+    int* err = nullptr;   // device flag of a timed-out wait (the owner's, else allocated on first use)
     // the list engine's lists (FP64 applies), shared by every column bucket
     struct Lists {
         bool ready = false;
         DevBook book;
         SLPart restrict_, ct, kept, dense, core, c, prolong;
         std::vector<SLPart> fwd, bwd;
+        // rounds [narrow_lo, n_rounds) run as one launch per direction (k_rounds)
+        uint32_t narrow_lo = 0;
+        uint32_t fwd_lo = 0, fwd_hi = 0, bwd_lo = 0, bwd_hi = 0;   // their rows
+        RDev fwd_narrow{}, bwd_narrow{};
+        size_t fwd_smem = 0, bwd_smem = 0;
     } lists;
 };
 
@@ -659,6 +665,81 @@ namespace {
 // pinned to those roundings in the directions the design does not determine.
 bool use_lists(const Tuning& t) {
     return t.warp_ranges == 1 && t.segthread && !t.vector_rows && t.wide_mean_len == UINT32_MAX;
+}
+
+// The suffix of rounds that k_rounds takes: each of them has to cost one block
+// less than a launch of its own.  A pass takes about 0.9 us and the block's
+// copies run at about 100 GB/s; a round's own launch takes 4.5 to 6.5 us
+// whatever its size.  The column's reduced vector, the
+// pass list and the stages have to fit in shared memory.
+constexpr size_t RP_SMEM_CAP = 220 * 1024;
+void plan_narrow_rounds(SchwarzUser& U, const SchwarzHost& H) {
+    auto& L = U.lists;
+    const uint32_t nr = H.n_rounds;
+    L.narrow_lo = nr;
+    if (!U.tuning.fuse_rounds || nr == 0) return;
+    auto bytes = [&](size_t n_pass) {
+        return RP_STAGES * sizeof(RStage) + n_pass * sizeof(RPass) + ((size_t)H.n_red + 1) * sizeof(double);
+    };
+    auto fwd = [&](NarrowRounds& N, uint32_t r) {
+        return N.add(H.fwd_ptr.data(), H.fwd_col.data(), H.fwd_val.data(), H.fwd_row.data(), H.fwd_round_ptr[r],
+                     H.fwd_round_ptr[r + 1], H.n_red);
+    };
+    auto bwd = [&](NarrowRounds& N, uint32_t r) {
+        return N.add(H.bwd_ptr.data(), H.bwd_col.data(), H.bwd_val.data(), H.bwd_row.data(), H.bwd_round_ptr[r],
+                     H.bwd_round_ptr[r + 1], H.n_red);
+    };
+    uint32_t lo = nr;
+    size_t nf = 0, nb = 0;
+    while (lo > 0 && bytes(nf + nb) <= RP_SMEM_CAP) {
+        // (a round this large is not worth packing to find out)
+        if (H.fwd_round_ptr[lo] - H.fwd_round_ptr[lo - 1] > 16 * RP_WARPS * RP_SLICE) break;
+        NarrowRounds f, b;
+        if (!fwd(f, lo - 1) || !bwd(b, lo - 1)) break;
+        auto us = [](const NarrowRounds& N) { return 0.9 * (double)N.pass.size() + 12e-5 * (double)N.val.size(); };
+        if (us(f) >= 4.5 || us(b) >= 4.5 || bytes(nf + f.pass.size()) > RP_SMEM_CAP ||
+            bytes(nb + b.pass.size()) > RP_SMEM_CAP)
+            break;
+        nf += f.pass.size();
+        nb += b.pass.size();
+        --lo;
+    }
+    if (nr - lo < 2) return;   // one round is one launch either way
+    NarrowRounds f, b;
+    for (uint32_t r = lo; r < nr; ++r) fwd(f, r);
+    for (uint32_t r = nr; r-- > lo;) bwd(b, r);
+    auto upload = [&](const NarrowRounds& N) {
+        static_assert(sizeof(RSlice) == sizeof(uint2), "slices are read as uint2");
+        RDev d;
+        d.val = U.arena.upload(N.val);
+        d.col = U.arena.upload(N.col);
+        d.row = U.arena.upload(N.row);
+        d.slice = reinterpret_cast<const uint2*>(U.arena.upload(N.slice));
+        d.pass = U.arena.upload(N.pass);
+        d.n_pass = (uint32_t)N.pass.size();
+        return d;
+    };
+    L.fwd_narrow = upload(f);
+    L.bwd_narrow = upload(b);
+    L.fwd_smem = bytes(f.pass.size());
+    L.bwd_smem = bytes(b.pass.size());
+    L.narrow_lo = lo;
+    L.fwd_lo = H.fwd_round_ptr[lo];
+    L.fwd_hi = H.fwd_round_ptr[nr];
+    L.bwd_lo = H.bwd_round_ptr[lo];
+    L.bwd_hi = H.bwd_round_ptr[nr];
+    // the shared-memory ceiling of the kernels, once per device
+    static std::mutex mu;
+    static std::vector<int> done;
+    std::lock_guard<std::mutex> g(mu);
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    if (std::find(done.begin(), done.end(), dev) != done.end()) return;
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    for (auto k : {k_rounds<1, false>, k_rounds<2, false>, k_rounds<4, false>, k_rounds<8, false>, k_rounds<1, true>,
+                   k_rounds<2, true>, k_rounds<4, true>, k_rounds<8, true>})
+        CK(cudaFuncSetAttribute(k, attr, (int)RP_SMEM_CAP));
+    done.push_back(dev);
 }
 
 void ensure_lists(SchwarzUser& U, const within_preconditioner& P) {
@@ -683,6 +764,8 @@ void ensure_lists(SchwarzUser& U, const within_preconditioner& P) {
                               SL_TARGET_BLOCKS));
     }
     L.book.upload(U.arena, b);
+    if (!U.err) U.err = U.arena.alloc<int>(1);
+    plan_narrow_rounds(U, H);
     L.ready = true;
 }
 
@@ -769,18 +852,6 @@ void ensure_tile_plans(SchwarzUser& U, const within_preconditioner& P, int K) {
     kp.fwd_thread = round_thread(H.fwd_round_ptr, H.fwd_ptr);
     kp.bwd_thread = round_thread(H.bwd_round_ptr, H.bwd_ptr);
     kp.plans = true;
-}
-
-// The rounds that run as one single-block launch per direction.
-void ensure_fused_rounds(SchwarzUser& U, const within_preconditioner& P, int K) {
-    KPlans& kp = U.kp[kidx(K)];
-    const SchwarzHost& H = P.host;
-    Arena& A = U.arena;
-    const bool segt_on = U.tuning.segthread;
-    auto short_round = [&](const std::vector<uint32_t>& rptr, const std::vector<uint32_t>& ptr, uint32_t r) {
-        const uint32_t m = rptr[r + 1] - rptr[r];
-        return m == 0 || seg_max_len(ptr.data() + rptr[r], m) <= SEGT_MAX_LEN;
-    };
     // the fused tail: the longest suffix of rounds that are one-thread rounds
     // in both directions with at most RF_MAX_ROWS rows (WITHIN_FUSE_ROUNDS=0: none)
     {
@@ -790,8 +861,8 @@ void ensure_fused_rounds(SchwarzUser& U, const within_preconditioner& P, int K) 
         auto ok = [&](uint32_t r) {
             const uint32_t fr = H.fwd_round_ptr[r + 1] - H.fwd_round_ptr[r];
             const uint32_t br = H.bwd_round_ptr[r + 1] - H.bwd_round_ptr[r];
-            return fr <= RF_MAX_ROWS && br <= RF_MAX_ROWS && short_round(H.fwd_round_ptr, H.fwd_ptr, r) &&
-                   short_round(H.bwd_round_ptr, H.bwd_ptr, r);
+            return (fr == 0 || kp.fwd_thread[r]) && (br == 0 || kp.bwd_thread[r]) && fr <= RF_MAX_ROWS &&
+                   br <= RF_MAX_ROWS;
         };
         while (fuse_on && lo > 0 && ok(lo - 1)) --lo;
         if (nr - lo >= 2) {
@@ -815,7 +886,6 @@ KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K
     Arena& A = U.arena;
     if (use_lists(U.tuning)) ensure_lists(U, P);
     else ensure_tile_plans(U, P, K);
-    ensure_fused_rounds(U, P, K);
     size_t nl = H.glob.size(), nr = H.n_red, ns = H.n_sub;
     kp.w.rl = A.alloc<double>(nl * K);
     kp.w.sl = A.alloc<double>(nl * K);
@@ -891,11 +961,19 @@ void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, c
             launch_sl<SlCt<K>, K>({{S}}, b, L.ct, P.ct_ptr, skip, st);
             launch_sl<SlKeptSum<K>, K>({{S}}, b, L.kept, S.kept_ptr, skip, st);
             if (P.has_dense) launch_sl<SlDense<K>, K>({{S}}, b, L.dense, P.dense_ptr, skip, st);
-            for (uint32_t q = 0; q < r_fwd_end; ++q) launch_sl<SlFwd<K>, K>({{S}}, b, L.fwd[q], P.fwd_ptr, skip, st);
-            fused_rounds(false);
+            for (uint32_t q = 0; q < L.narrow_lo; ++q) launch_sl<SlFwd<K>, K>({{S}}, b, L.fwd[q], P.fwd_ptr, skip, st);
+            if (L.fwd_narrow.n_pass) {
+                launch_k(k_rounds<K, false>, K, RP_THREADS + 32, L.fwd_smem, st, S, L.fwd_narrow, L.fwd_lo, L.fwd_hi,
+                         P.host.n_red, U.err, skip);
+                ++g_launches;
+            }
             if (P.has_core) launch_sl<SlCore<K>, K>({{S}}, b, L.core, P.core_ptr, skip, st);
-            fused_rounds(true);
-            for (uint32_t q = r_fwd_end; q-- > 0;) launch_sl<SlBwd<K>, K>({{S}}, b, L.bwd[q], P.bwd_ptr, skip, st);
+            if (L.bwd_narrow.n_pass) {
+                launch_k(k_rounds<K, true>, K, RP_THREADS + 32, L.bwd_smem, st, S, L.bwd_narrow, L.bwd_lo, L.bwd_hi,
+                         P.host.n_red, U.err, skip);
+                ++g_launches;
+            }
+            for (uint32_t q = L.narrow_lo; q-- > 0;) launch_sl<SlBwd<K>, K>({{S}}, b, L.bwd[q], P.bwd_ptr, skip, st);
             launch_sl<SlC<K>, K>({{S}}, b, L.c, P.c_ptr, skip, st);
             launch_sl<SlMean<K>, K>({{S}}, b, L.restrict_, S.loc_ptr, skip, st);
             launch_sl<SlProlong<K>, K>({{S}, z}, b, L.prolong, P.dof_ptr, skip, st);
@@ -1920,7 +1998,7 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
     CK(cudaMemcpyAsync(b2, w.st + 8, sizeof(ColState) * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(&werr, s.sweep_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (werr) throw WError(ERR_CUDA, "staged gather: a bulk copy into shared memory did not complete within 1 s");
+    if (werr) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
     for (int k = 0; k < 8; ++k) fin[k] = a[k].itn >= b2[k].itn ? a[k] : b2[k];
     if (stop_out)
         for (uint32_t k = 0; k < k_used; ++k) stop_out[k] = fin[k].stop;
@@ -2230,7 +2308,7 @@ void run_mixed(within_solver& s, const double* Y, uint32_t k_used, double tol, u
     int werr = 0;
     CK(cudaMemcpyAsync(&werr, s.sweep_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (werr) throw WError(ERR_CUDA, "staged gather: a bulk copy into shared memory did not complete within 1 s");
+    if (werr) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
     const double t_end = now_s();
     if (stats)
         for (uint32_t k = 0; k < k_used; ++k) {
@@ -2350,6 +2428,7 @@ within_solver* make_solver(const within_design* d, const double* weights, const 
     CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     s->sweep_err = s->arena.alloc<int>(1);
     s->schwarz.tuning = resolve_tuning(tuning);
+    s->schwarz.err = s->sweep_err;
     pdl_setup(device);
     std::vector<EffectIn> effs;
     for (size_t e = 0; e < d->levels.size(); ++e) {
@@ -3102,7 +3181,7 @@ int within_solver_operator_apply(within_solver* s, const double* x_dev, double* 
             CK(cudaStreamSynchronize(st));
             int e = 0;
             CK(cudaMemcpy(&e, s->sweep_err, sizeof(int), cudaMemcpyDeviceToHost));
-            if (e) throw WError(ERR_CUDA, "staged gather: a bulk copy into shared memory did not complete within 1 s");
+            if (e) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
         }
     });
 }
@@ -3325,6 +3404,7 @@ int within_preconditioner_apply(const within_preconditioner* pc, const double* x
         auto* p = const_cast<within_preconditioner*>(pc);
         set_device(p->device);
         cudaStream_t st = stream ? (cudaStream_t)stream : nullptr;
+        int werr = 0;
         if (p->kind == 2) {
             launch_k(k_diag_apply<1>, grid_for(p->n, 256, 148 * 8), 256, 0, st, p->n, p->inv_diag, x_dev, y_dev, nullptr);
             ++g_launches;
@@ -3335,9 +3415,12 @@ int within_preconditioner_apply(const within_preconditioner* pc, const double* x
                 p->standalone->tuning = resolve_tuning(nullptr);
             }
             schwarz_apply<1>(*p, *p->standalone, x_dev, y_dev, nullptr, st);
+            if (p->standalone->lists.fwd_narrow.n_pass)
+                CK(cudaMemcpyAsync(&werr, p->standalone->err, sizeof(int), cudaMemcpyDeviceToHost, st));
         }
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(st));
+        if (werr) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
     });
 }
 
