@@ -1443,6 +1443,13 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
     uint64_t rpr = (n + G - 1) / G;
     rpr = std::max<uint64_t>(min_range, (rpr + CH - 1) / CH * CH);
     rp.rows_per_range = (uint32_t)rpr;
+    // only the blocks whose ranges hold rows: on 2,003 rows the last block of a
+    // full grid added 444 blocks' bins for 31 of the sweep's 34 us
+    {
+        const uint64_t per_block = rpr * (G / (uint64_t)rk.grid);
+        rk.grid = (int)std::min<uint64_t>((uint64_t)rk.grid, (n + per_block - 1) / per_block);
+        G = (uint64_t)rk.grid * (per_block / rpr);
+    }
     std::vector<RwFix> fixes;
     size_t first_prob = 0;
     for (int t = 0; t < Q; ++t) {
