@@ -64,7 +64,6 @@ struct Reparam {
     std::vector<TermR> terms;
     std::vector<uint64_t> unidentified;   // (term, level, column) triples
     bool active() const { return !terms.empty(); }
-    void back_transform(double* x) const;
 };
 Reparam build_reparam(HostDesign& d, const double* weights_internal);
 

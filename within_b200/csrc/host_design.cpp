@@ -316,29 +316,6 @@ Reparam build_reparam(HostDesign& d, const double* w) {
     return out;
 }
 
-// reparam.rs:173-194
-void Reparam::back_transform(double* x) const {
-    for (const auto& t : terms) {
-        const size_t v = t.slope_cols.size();
-        std::vector<double> b(v);
-        for (size_t l = 0; l < t.w.size(); ++l) {
-            const auto& wl = t.w[l];
-            if (wl.empty()) continue;
-            std::fill(b.begin(), b.end(), 0.0);
-            for (size_t k = 0; k * v < wl.size(); ++k) {
-                double bk = x[t.offset + (size_t)t.slope_cols[k] * t.n_levels + l];
-                for (size_t j = 0; j < v; ++j) b[j] += wl[k * v + j] * bk;
-            }
-            for (size_t j = 0; j < v; ++j) x[t.offset + (size_t)t.slope_cols[j] * t.n_levels + l] = b[j];
-            if (t.intercept_col >= 0) {
-                double s = 0;
-                for (size_t j = 0; j < v; ++j) s += b[j] * t.center[l][j];
-                x[t.offset + (size_t)t.intercept_col * t.n_levels + l] -= s;
-            }
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Tile plan of one segmented-reduction problem (see segreduce.cuh).
 void HostPlan::add(uint32_t problem, const uint32_t* ptr, uint32_t n_seg, int T) {

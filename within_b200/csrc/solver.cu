@@ -1107,6 +1107,7 @@ struct within_solver {
     // the scan sweep's ranges for the FP32 normal operator where rsw is cut
     // for the column-lane sweep (built for mixed precision only; run sums shared)
     RowSweepK rsw_f[4];
+    std::vector<BackTerm> back;   // slope terms' back-transform (x leaves the whitened basis)
     int* sweep_err = nullptr;   // device flag of a timed-out wait in a sweep outside the LSMR loop
     // per column bucket, the LSMR step's operator path:
     // 0 gather + full segmented-reduction scatter, 2 warp-range row sweep (rowsweep.cuh)
@@ -2390,6 +2391,15 @@ void dispatch_solve(within_solver& s, const double* Y_dev, uint64_t k, double to
     }
 }
 
+// X (column-major n_dofs x k, device) out of the slope terms' whitened basis.
+void back_transform(within_solver& s, uint64_t k, double* X, cudaStream_t st) {
+    for (const BackTerm& b : s.back) {
+        launch_k(k_back_transform, grid_for((uint64_t)b.n_levels * k, 256, 148 * 8), 256, 0, st, b, s.n_dofs,
+                 (uint32_t)k, X);
+        ++g_launches;
+    }
+}
+
 void validate_opts(const within_lsmr_options* o, double& tol, uint64_t& maxiter, uint64_t& local_size) {
     tol = 1e-8;
     maxiter = 1000;
@@ -2590,6 +2600,28 @@ within_solver* make_solver(const within_design* d, const double* weights, const 
     }
     // the rest of the design operator on the device
     PhaseTrace pt_op("design upload and scatter orders");
+    for (const Reparam::TermR& t : s->reparam.terms) {
+        BackTerm b{};
+        b.offset = t.offset;
+        b.n_levels = t.n_levels;
+        b.n_slopes = (uint32_t)t.slope_cols.size();
+        b.intercept = t.intercept_col;
+        for (size_t j = 0; j < t.slope_cols.size(); ++j) b.slope_col[j] = t.slope_cols[j];
+        std::vector<uint32_t> ptr(1, 0);
+        std::vector<double> wv, cv((size_t)t.n_levels * b.n_slopes, 0.0);
+        for (size_t l = 0; l < t.n_levels; ++l) {
+            if (l < t.w.size() && !t.w[l].empty()) {
+                wv.insert(wv.end(), t.w[l].begin(), t.w[l].end());
+                if (t.intercept_col >= 0)   // read for the intercept only
+                    std::copy(t.center[l].begin(), t.center[l].end(), cv.begin() + l * b.n_slopes);
+            }
+            ptr.push_back((uint32_t)wv.size());
+        }
+        b.w_ptr = A.upload(ptr);
+        b.w = A.upload(wv);
+        b.center = A.upload(cv);
+        s->back.push_back(b);
+    }
     if (weights) {
         std::vector<double> sw(w);
         for (double& x : sw) x = std::sqrt(x);
@@ -2814,13 +2846,10 @@ void host_solve(within_solver& s, const double* Y, uint64_t k, const within_lsmr
         io.h2d(dY, Y, k * n * sizeof(double));
     }
     dispatch_solve(s, dY, k, tol, maxiter, X ? dX : nullptr, Dm ? dD : nullptr, stats, s.stream, ls);
+    if (X) back_transform(s, k, dX, s.stream);
     PhaseTrace pt_out("device -> host copy of the results");
     if (Dm) io.d2h(Dm, dD, k * n * sizeof(double));
-    if (X) {
-        io.d2h(X, dX, k * nd * sizeof(double));
-        if (s.reparam.active())
-            for (uint64_t j = 0; j < k; ++j) s.reparam.back_transform(X + j * nd);
-    }
+    if (X) io.d2h(X, dX, k * nd * sizeof(double));
 }
 
 // Runs fn(i) for i in [0, n) on `threads` host threads (device `dev` current
@@ -3103,12 +3132,8 @@ int within_solver_solve_batch_device(within_solver* s, const double* Y_dev, uint
         set_device(s->device);
         cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
         dispatch_solve(*s, Y_dev, k, tol, maxiter, X_dev, D_dev, stats, st, ls);
-        if (X_dev && s->reparam.active()) {
-            std::vector<double> hx(k * s->n_dofs);
-            CK(cudaMemcpyAsync(hx.data(), X_dev, hx.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            for (uint64_t j = 0; j < k; ++j) s->reparam.back_transform(hx.data() + j * s->n_dofs);
-            CK(cudaMemcpyAsync(X_dev, hx.data(), hx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+        if (X_dev && !s->back.empty()) {
+            back_transform(*s, k, X_dev, st);
             CK(cudaStreamSynchronize(st));
         }
     });
@@ -3139,12 +3164,8 @@ int within_solver_solve_batch_device_ext(within_solver* s, const double* Y_dev, 
             throw WError(ERR_UNSUPPORTED, "warm starts are supported for designs without slope terms");
         cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
         dispatch_solve(*s, Y_dev, k, tol, maxiter, X_dev, D_dev, stats, st, ls, e, stop_reason);
-        if (X_dev && s->reparam.active()) {
-            std::vector<double> hx(k * s->n_dofs);
-            CK(cudaMemcpyAsync(hx.data(), X_dev, hx.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            for (uint64_t j = 0; j < k; ++j) s->reparam.back_transform(hx.data() + j * s->n_dofs);
-            CK(cudaMemcpyAsync(X_dev, hx.data(), hx.size() * sizeof(double), cudaMemcpyHostToDevice, st));
+        if (X_dev && !s->back.empty()) {
+            back_transform(*s, k, X_dev, st);
             CK(cudaStreamSynchronize(st));
         }
     });
