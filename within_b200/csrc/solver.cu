@@ -1097,7 +1097,7 @@ struct within_solver {
         // staged sweep (tsweep.cuh): used for the FP64 adjoint and LSMR-step modes
         bool ts = false;
         TsSlots ts_slots{};
-        int ts_nq = 0;
+        int ts_nq = 0, ts_ns = 0;            // terms, slope columns
         size_t ts_smem = 0;
         // column-lane sweep (csweep.cuh): the FP64 modes of K = 2, 4, 8
         bool cs = false;
@@ -1265,7 +1265,22 @@ TsKernel ts_pick_q(int nq, int nrun, int nhist) {
         default: return ts_pick_r<MODE, 3, WTD>(nrun, nhist);
     }
 }
-TsKernel ts_kernel(int mode, int nq, int nrun, int nhist, bool wtd) {
+// ... and of designs with one slope column, one run term and at most one
+// histogram term
+template <int MODE, bool WTD>
+TsKernel ts_pick_slope(int nq, int nhist) {
+    if (nhist == 0)
+        return nq == 1   ? (TsKernel)k_tsweep<1, MODE, 1, 1, 0, WTD, 1>
+               : nq == 2 ? (TsKernel)k_tsweep<1, MODE, 2, 1, 0, WTD, 1>
+                         : (TsKernel)k_tsweep<1, MODE, 3, 1, 0, WTD, 1>;
+    return nq == 2 ? (TsKernel)k_tsweep<1, MODE, 2, 1, 1, WTD, 1> : (TsKernel)k_tsweep<1, MODE, 3, 1, 1, WTD, 1>;
+}
+TsKernel ts_kernel(int mode, int nq, int nrun, int nhist, bool wtd, int ns = 0) {
+    if (ns) {
+        if (nq < 1 || nq > TS_MAXQ || nrun != 1 || nhist < 0 || nhist > 1 || nrun + nhist > nq) return nullptr;
+        if (mode == 0) return wtd ? ts_pick_slope<0, true>(nq, nhist) : ts_pick_slope<0, false>(nq, nhist);
+        return wtd ? ts_pick_slope<1, true>(nq, nhist) : ts_pick_slope<1, false>(nq, nhist);
+    }
     if (nq < 1 || nq > TS_MAXQ || nrun < 1 || nrun > RW_MAX_RUN || nhist < 0 || nhist > RW_MAX_HIST) return nullptr;
     if (mode == 0) return wtd ? ts_pick_q<0, true>(nq, nrun, nhist) : ts_pick_q<0, false>(nq, nrun, nhist);
     return wtd ? ts_pick_q<1, true>(nq, nrun, nhist) : ts_pick_q<1, false>(nq, nrun, nhist);
@@ -1402,11 +1417,22 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
             nhist += cls[t] == CLS_HIST;
             if (cls[t] == CLS_HIST) nbk += (int)D.terms[t].n_levels;
         }
-        const bool ok = K == 1 && simple && Q <= TS_MAXQ && nrun >= 1 && s.schwarz.tuning.staged;
-        const size_t sm = ts_smem_bytes<K>(nbk, nhist, Q, s.op.sqrt_w != nullptr);
+        // one slope column: terms of up to two columns (intercept, slope), one run
+        // term and at most one histogram term (2,000,000 rows, firm intercept and
+        // slope, years: 70 us in the generic sweep, 38 us here)
+        bool one_slope = D.loads.size() == 1 && nrun == 1 && nhist <= 1;
+        nbk = 0;
+        for (int t = 0; t < Q; ++t) {
+            one_slope = one_slope && D.terms[t].cols.size() <= 2;
+            if (cls[t] == CLS_HIST) nbk += (int)(D.terms[t].n_levels * D.terms[t].cols.size());
+        }
+        const bool ok = K == 1 && (simple || one_slope) && Q <= TS_MAXQ && nrun >= 1 && s.schwarz.tuning.staged;
+        const size_t sm = simple ? ts_smem_bytes<K>(nbk, nhist, Q, s.op.sqrt_w != nullptr)
+                                 : ts_ring_offset<K>(nbk, nhist);
         if (ok && sm <= TS_SMEM_CAP) {
             rk.ts = true;
             rk.ts_nq = Q;
+            rk.ts_ns = simple ? 0 : 1;
             rk.ts_smem = sm;
             int k = 0;
             for (int t = 0; t < Q; ++t)
@@ -1596,8 +1622,9 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
                         for (int nrun = 1; nrun <= RW_MAX_RUN; ++nrun)
                             for (int nhist = 0; nhist <= RW_MAX_HIST; ++nhist)
                                 for (int wtd = 0; wtd < 2; ++wtd)
-                                    if (auto f = ts_kernel(mode, nq, nrun, nhist, wtd != 0))
-                                        CK(cudaFuncSetAttribute(f, attr, (int)TS_SMEM_CAP));
+                                    for (int ns = 0; ns < 2; ++ns)
+                                        if (auto f = ts_kernel(mode, nq, nrun, nhist, wtd != 0, ns))
+                                            CK(cudaFuncSetAttribute(f, attr, (int)TS_SMEM_CAP));
             } else {
                 const int cs_cap = (int)cs_smem_bytes(RW_MAX_BUCKETS);
                 CK(cudaFuncSetAttribute(k_csweep<K, 0, false>, attr, cs_cap));
@@ -1672,7 +1699,7 @@ void launch_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const OpPar
     if constexpr (K == 1 && (MODE == 0 || MODE == 1) && sizeof(T) == 8) {
         // bulk copies read u from 16-byte aligned chunk starts
         if (rk.ts && ((uintptr_t)u & 15) == 0 && (MODE == 1 || !skip)) {
-            TsKernel f = ts_kernel(MODE, rk.ts_nq, rp.n_run, rp.n_hist, op.sqrt_w != nullptr);
+            TsKernel f = ts_kernel(MODE, rk.ts_nq, rp.n_run, rp.n_hist, op.sqrt_w != nullptr, rk.ts_ns);
             if (f) {
                 rp.hist_private = 1;
                 int* e = err ? err : (ctl ? &ctl->err : s.sweep_err);

@@ -89,7 +89,21 @@ __device__ __forceinline__ void ts_issue(char* stage, uint64_t* bar, const OpPar
     if constexpr (WTD) bulk_g2s(stage + NQ * RG::CODE_B + RG::U_B, p.sqrt_w + c0, w_b, bar);
 }
 
-template <int K, int MODE, int NQ, int NRUN, int NHIST, bool WTD>
+// The loadings of a design with one slope column, per lane: column c of a
+// term loads 1 (intercept) or the slope.
+template <int R>
+__device__ __forceinline__ double ts_load(bool slope, const double (&sl)[R], int r) {
+    return slope ? sl[r] : 1.0;
+}
+
+// NS = 0: intercept-only, staged.  NS = 1: the design has one slope column, and
+// its terms up to two columns each (intercept, slope).  Its streams (codes, u,
+// sqrt(w), slope) are plain vector loads requested one chunk ahead instead: a
+// ring of 4 KB chunks beside the wider bins would leave eight warps per SM.
+// 2,000,000 rows, weighted, firm intercept and slope and 30 years: LSMR step 70 ->
+// 38 us, adjoint 57 -> 32 us against the generic sweep, whose loops over terms and
+// columns are not unrolled and which reads the slope again for every use.
+template <int K, int MODE, int NQ, int NRUN, int NHIST, bool WTD, int NS = 0>
 __global__ void __launch_bounds__(RW_THREADS, TS_BLOCKS_PER_SM)
 k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, double* __restrict__ u,
          ColState* cur, Ctl* ctl, int* err) {
@@ -136,6 +150,16 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
     const uint32_t r1 = (uint32_t)min(r0w + rw.rows_per_range, (uint64_t)p.n);
     const uint32_t n_chunks = (r1 - r0 + CH - 1) / CH;
 
+    // columns of each term and which of them load the slope (one column, an intercept, at NS = 0)
+    constexpr int MC = NS ? 2 : 1;
+    int ncol[NQ];
+    bool slope[NQ][MC];
+#pragma unroll
+    for (int t = 0; t < NQ; ++t) {
+        ncol[t] = NS ? p.ncol[t] : 1;
+#pragma unroll
+        for (int c = 0; c < MC; ++c) slope[t][c] = NS && c < ncol[t] && p.load[t][c] >= 0;
+    }
     // slot terms (warp-uniform)
     int st_run[NRUN], st_hist[NHIST > 0 ? NHIST : 1];
 #pragma unroll
@@ -144,14 +168,16 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
     for (int h = 0; h < NHIST; ++h) st_hist[h] = sl.term[NRUN + h];
 
     // run-term state (warp-uniform except the carry, which every lane holds)
-    double carry[NRUN][K];
+    double carry[NRUN][MC][K];
     bool started[NRUN];      // the open run's head lies in this range
     uint32_t prevc[NRUN];    // code of the row before the chunk
     uint32_t heads[NRUN];    // heads seen in the range before the chunk
 #pragma unroll
     for (int j = 0; j < NRUN; ++j) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) carry[j][k] = 0.0;
+        for (int c = 0; c < MC; ++c)
+#pragma unroll
+            for (int k = 0; k < K; ++k) carry[j][c][k] = 0.0;
         started[j] = false;
         heads[j] = 0;
         prevc[j] = 0u;
@@ -159,7 +185,7 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
     }
 
     // ring set-up and prologue (lane 0 issues, the warp waits)
-    if (lane == 0) {
+    if (NS == 0 && lane == 0) {
         for (int s = 0; s < TS_STAGES; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
     }
@@ -168,32 +194,61 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
         const uint32_t c0 = r0 + j * CH;
         return min((uint32_t)CH, r1 - c0) & ~3u;
     };
-    if (lane == 0)
+    if (NS == 0 && lane == 0)
         for (uint32_t j = 0; j < (uint32_t)TS_STAGES && j < n_chunks; ++j)
             ts_issue<K, NQ, WTD, double>(ring + j * RG::STAGE_B, &bars[j], p, u, r0 + j * CH, bulk_rows(j));
     bool failed = false;
     uint32_t failed_at = 0;
+    // NS > 0: the next chunk's rows of this lane
+    struct Rows {
+        uint32_t cd[NQ][R];
+        double u[R * K], w[R], s[R];
+    } nx;
+    auto fetch = [&](uint32_t j) {
+        const uint32_t row0 = r0 + j * CH + (uint32_t)lane * R;
+        const int nr = row0 < r1 ? (int)min((uint32_t)R, r1 - row0) : 0;
+#pragma unroll
+        for (int t = 0; t < NQ; ++t) rw_load_codes<R>(p.codes[t], row0, nr, nx.cd[t]);
+        rw_load_vals<R * K, double>(u + (size_t)row0 * K, nr * K, nx.u);
+        if constexpr (WTD) rw_load_vals<R, double>(p.sqrt_w + row0, nr, nx.w);
+        rw_load_vals<R, double>(p.loads[0] + row0, nr, nx.s);
+    };
+    if constexpr (NS > 0)
+        if (n_chunks) fetch(0);
 
     for (uint32_t j = 0; j < n_chunks; ++j) {
         const int stg = (int)(j % TS_STAGES);
-        const uint32_t par = (j / TS_STAGES) & 1u;
-        const bool landed = mbar_wait_bounded(&bars[stg], par);
-        if (!__all_sync(FULL, landed)) {   // warp-uniform: every lane leaves together
-            failed = true;
-            failed_at = j;
-            break;
+        if constexpr (NS == 0) {
+            const uint32_t par = (j / TS_STAGES) & 1u;
+            const bool landed = mbar_wait_bounded(&bars[stg], par);
+            if (!__all_sync(FULL, landed)) {   // warp-uniform: every lane leaves together
+                failed = true;
+                failed_at = j;
+                break;
+            }
         }
         const char* sp = ring + stg * RG::STAGE_B;
         const uint32_t c0 = r0 + j * CH;
         const uint32_t nbulk = bulk_rows(j);
         const uint32_t row0 = c0 + (uint32_t)lane * R;
         const int nr = row0 < r1 ? (int)min((uint32_t)R, r1 - row0) : 0;
-        const bool in_smem = row0 + R <= c0 + nbulk;   // this lane's rows were copied
-        // ---- this lane's rows: codes of every term, u (K columns), sqrt(w)
+        const bool in_smem = NS ? nr == R : row0 + R <= c0 + nbulk;   // this lane's rows were copied (NS: are whole)
+        // ---- this lane's rows: codes of every term, u (K columns), sqrt(w), the slope
         uint32_t cd[NQ][R];
         double uin[R * K];
-        double wv[R];
-        if (in_smem) {
+        double wv[R], sl[R];
+        if constexpr (NS > 0) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+#pragma unroll
+                for (int t = 0; t < NQ; ++t) cd[t][r] = nx.cd[t][r];
+#pragma unroll
+                for (int k = 0; k < K; ++k) uin[r * K + k] = nx.u[r * K + k];
+                if constexpr (WTD) wv[r] = nx.w[r];
+                sl[r] = nx.s[r];
+            }
+            if (j + 1 < n_chunks) fetch(j + 1);
+        } else if (in_smem) {
 #pragma unroll
             for (int t = 0; t < NQ; ++t) {
                 const uint32_t* sc = reinterpret_cast<const uint32_t*>(sp + t * RG::CODE_B) + lane * R;
@@ -233,13 +288,14 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
                 for (int r = 0; r < R; ++r) wv[r] = r < nr ? __ldg(p.sqrt_w + row0 + r) : 0.0;
             }
         }
-        if constexpr (!WTD) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) wv[r] = 1.0;
+        for (int r = 0; r < R; ++r) {
+            if constexpr (!WTD) wv[r] = 1.0;
+            if constexpr (NS == 0) sl[r] = 0.0;
         }
         __syncwarp();
         // every lane has its rows in registers: the stage refills with chunk j + TS_STAGES
-        if (lane == 0 && j + TS_STAGES < n_chunks) {
+        if (NS == 0 && lane == 0 && j + TS_STAGES < n_chunks) {
             fence_proxy_async_smem();
             ts_issue<K, NQ, WTD, double>(ring + stg * RG::STAGE_B, &bars[stg], p, u, c0 + TS_STAGES * CH,
                                          bulk_rows(j + TS_STAGES));
@@ -260,14 +316,19 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
                 for (int k = 0; k < K; ++k) s[r][k] = 0.0;
 #pragma unroll
             for (int t = 0; t < NQ; ++t) {
-                const size_t col = p.off[t];
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (r >= nr) continue;
-                    double xg[K];
-                    ldgk<K, double>(v + (col + cd[t][r]) * K, xg);
+                for (int cc = 0; cc < MC; ++cc) {
+                    if (cc >= ncol[t]) break;
+                    const size_t col = (size_t)p.off[t] + (size_t)cc * p.L[t];
 #pragma unroll
-                    for (int k = 0; k < K; ++k) s[r][k] += xg[k];
+                    for (int r = 0; r < R; ++r) {
+                        if (r >= nr) continue;
+                        double xg[K];
+                        ldgk<K, double>(v + (col + cd[t][r]) * K, xg);
+#pragma unroll
+                        for (int k = 0; k < K; ++k)
+                            s[r][k] += NS ? xg[k] * ts_load<R>(slope[t][cc], sl, r) : xg[k];
+                    }
                 }
             }
             double outv[R * K];
@@ -308,9 +369,22 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
 #pragma unroll
                 for (int q = 1; q < NQ; ++q)
                     if (t == q) c = cd[q][r];
-                const int bk = b0 + (int)c;
 #pragma unroll
-                for (int k = 0; k < K; ++k) pbins[(bk * K + k) * 32 + lane] += b[r][k];
+                for (int cc = 0; cc < MC; ++cc) {
+                    int nc = ncol[0];
+                    bool sc = slope[0][cc];
+#pragma unroll
+                    for (int q = 1; q < NQ; ++q)
+                        if (t == q) {
+                            nc = ncol[q];
+                            sc = slope[q][cc];
+                        }
+                    if (cc >= nc) break;
+                    const int bk = b0 + (int)c * nc + cc;
+#pragma unroll
+                    for (int k = 0; k < K; ++k)
+                        pbins[(bk * K + k) * 32 + lane] += NS ? ts_load<R>(sc, sl, r) * b[r][k] : b[r][k];
+                }
             }
         }
 
@@ -338,39 +412,15 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
                 hd[r] = r < nr && (row0 + r == 0 || c[r] != pc);
                 lane_heads += hd[r] ? 1 : 0;
             }
-            // lane aggregate: sum since the lane's last head (or of the whole lane)
-            double sv[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) sv[k] = 0.0;
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int k = 0; k < K; ++k) sv[k] = hd[r] ? b[r][k] : sv[k] + b[r][k];
             const unsigned hm = __ballot_sync(FULL, lane_heads > 0);
             const unsigned lt = lanemask_lt();
             const int hl = 31 - __clz(hm & (lt | (1u << lane)));   // last lane <= lane with a head, or -1
             const int hl0 = hl < 0 ? 0 : hl;
-            // segmented inclusive scan over the lanes
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1)
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const double up = __shfl_up_sync(FULL, sv[k], d);
-                    if (lane - d >= hl0) sv[k] += up;
-                }
-            // the run open at the start of this lane's rows
             const bool exf = (hm & lt) != 0;
-            double run[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                double ex = __shfl_up_sync(FULL, sv[k], 1);
-                if (lane == 0) ex = 0.0;
-                run[k] = exf ? ex : carry[jr][k] + ex;
-            }
-            bool in_range = exf || started[jr];
+            const bool chunk_has_head = hm != 0;
             // heads before this lane within the chunk (ordinals of the runs of a non-direct term)
             // (the chunk's head count only matters to a term summed by run ordinal)
-            uint32_t ord = 0, chunk_heads = 0;
+            uint32_t ord0 = 0, chunk_heads = 0;
             if (!RR.direct) {
                 int before = 0;
 #pragma unroll
@@ -379,42 +429,90 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
                     before += __popc(bl & lt);
                     chunk_heads += (uint32_t)__popc(bl);
                 }
-                ord = __ldg(RR.range_base + g) + heads[jr] + (uint32_t)before;   // ordinal of the next head
+                ord0 = __ldg(RR.range_base + g) + heads[jr] + (uint32_t)before;   // ordinal of the next head
             }
-            // a head ends the run before it: a complete run (its head lies in this
-            // range), or the head partial of a run that started in an earlier range
+            int nc = ncol[0];
+            bool sc[MC];
+            uint32_t nlev = p.L[0];
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (hd[r]) {
-                    if (row0 + r > r0) {
-                        if (!in_range) {
+            for (int cc = 0; cc < MC; ++cc) sc[cc] = slope[0][cc];
 #pragma unroll
-                            for (int k = 0; k < K; ++k) RR.head[(size_t)g * K + k] = run[k];
-                        } else if (RR.direct) {
-                            const uint32_t lvl = r == 0 ? pc0 : c[r - 1];
-                            const size_t dof = (size_t)p.off[t] + lvl;
+            for (int q = 1; q < NQ; ++q)
+                if (t == q) {
+                    nc = ncol[q];
+                    nlev = p.L[q];
 #pragma unroll
-                            for (int k = 0; k < K; ++k) reinterpret_cast<double*>(rw.atu)[dof * K + k] = run[k];
-                        } else {
-#pragma unroll
-                            for (int k = 0; k < K; ++k) RR.run_sum[(size_t)(ord - 1) * K + k] = run[k];
-                        }
-                    }
-                    ++ord;
-                    in_range = true;
-#pragma unroll
-                    for (int k = 0; k < K; ++k) run[k] = b[r][k];
-                } else {
-#pragma unroll
-                    for (int k = 0; k < K; ++k) run[k] += b[r][k];
+                    for (int cc = 0; cc < MC; ++cc) sc[cc] = slope[q][cc];
                 }
-            }
-            // carry the open run into the next chunk
-            const bool chunk_has_head = hm != 0;
+            if constexpr (NS == 0) nc = 1;
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const double incl = __shfl_sync(FULL, sv[k], 31);
-                carry[jr][k] = chunk_has_head ? incl : carry[jr][k] + incl;
+            for (int cc = 0; cc < MC; ++cc) {
+                if (cc >= nc) break;
+                double val[R][K];
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int k = 0; k < K; ++k) val[r][k] = NS ? ts_load<R>(sc[cc], sl, r) * b[r][k] : b[r][k];
+                // lane aggregate: sum since the lane's last head (or of the whole lane)
+                double sv[K];
+#pragma unroll
+                for (int k = 0; k < K; ++k) sv[k] = 0.0;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int k = 0; k < K; ++k) sv[k] = hd[r] ? val[r][k] : sv[k] + val[r][k];
+                // segmented inclusive scan over the lanes
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const double up = __shfl_up_sync(FULL, sv[k], d);
+                        if (lane - d >= hl0) sv[k] += up;
+                    }
+                // the run open at the start of this lane's rows
+                double run[K];
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    double ex = __shfl_up_sync(FULL, sv[k], 1);
+                    if (lane == 0) ex = 0.0;
+                    run[k] = exf ? ex : carry[jr][cc][k] + ex;
+                }
+                bool in_range = exf || started[jr];
+                uint32_t ord = ord0;
+                // a head ends the run before it: a complete run (its head lies in this
+                // range), or the head partial of a run that started in an earlier range
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (hd[r]) {
+                        if (row0 + r > r0) {
+                            if (!in_range) {
+#pragma unroll
+                                for (int k = 0; k < K; ++k) RR.head[((size_t)g * nc + cc) * K + k] = run[k];
+                            } else if (RR.direct) {
+                                const uint32_t lvl = r == 0 ? pc0 : c[r - 1];
+                                const size_t dof = (size_t)p.off[t] + (size_t)cc * nlev + lvl;
+#pragma unroll
+                                for (int k = 0; k < K; ++k) reinterpret_cast<double*>(rw.atu)[dof * K + k] = run[k];
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < K; ++k) RR.run_sum[((size_t)(ord - 1) * nc + cc) * K + k] = run[k];
+                            }
+                        }
+                        ++ord;
+                        in_range = true;
+#pragma unroll
+                        for (int k = 0; k < K; ++k) run[k] = val[r][k];
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < K; ++k) run[k] += val[r][k];
+                    }
+                }
+                // carry the open run into the next chunk
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const double incl = __shfl_sync(FULL, sv[k], 31);
+                    carry[jr][cc][k] = chunk_has_head ? incl : carry[jr][cc][k] + incl;
+                }
             }
             started[jr] = started[jr] || chunk_has_head;
             heads[jr] += chunk_heads;
@@ -441,27 +539,32 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
             const uint32_t* cdp = p.codes[t];
             const uint32_t last = __ldg(cdp + r1 - 1);
             const bool cont = r1 < p.n && __ldg(cdp + r1) == last;
-            double* dst;
-            size_t idx;
-            if (!started[jr]) {
-                dst = RR.head;
-                idx = g;
-            } else if (cont) {
-                dst = RR.tail;
-                idx = g;
-            } else if (RR.direct) {
-                dst = reinterpret_cast<double*>(rw.atu);
-                idx = (size_t)p.off[t] + last;
-            } else {
-                dst = RR.run_sum;
-                idx = (size_t)__ldg(RR.range_base + g) + heads[jr] - 1;
-            }
+            const int nc = NS ? p.ncol[t] : 1;
 #pragma unroll
-            for (int k = 0; k < K; ++k) dst[idx * K + k] = carry[jr][k];
+            for (int cc = 0; cc < MC; ++cc) {
+                if (cc >= nc) break;
+                double* dst;
+                size_t idx;
+                if (!started[jr]) {
+                    dst = RR.head;
+                    idx = (size_t)g * nc + cc;
+                } else if (cont) {
+                    dst = RR.tail;
+                    idx = (size_t)g * nc + cc;
+                } else if (RR.direct) {
+                    dst = reinterpret_cast<double*>(rw.atu);
+                    idx = (size_t)p.off[t] + (size_t)cc * p.L[t] + last;
+                } else {
+                    dst = RR.run_sum;
+                    idx = ((size_t)__ldg(RR.range_base + g) + heads[jr] - 1) * nc + cc;
+                }
+#pragma unroll
+                for (int k = 0; k < K; ++k) dst[idx * K + k] = carry[jr][cc][k];
+            }
         }
     }
 
-    rw_finish<K, MODE, double, true>(p, rw, accn, act, cur, nullptr, 0);
+    rw_finish<K, MODE, double, NS == 0>(p, rw, accn, act, cur, nullptr, 0);
 }
 
 }  // namespace wgpu
