@@ -1260,8 +1260,8 @@ k_load_rhs(uint32_t n, uint32_t k_used, const double* __restrict__ Y, const uint
 template <int K>
 __global__ void __launch_bounds__(RED_THREADS)
 k_norm_b(uint32_t n, const double* __restrict__ b, const double* bmax, ColState* st, double tol,
-         long long maxiter, uint32_t k_used, Ctl* ctl, double* partials, unsigned* counter, int warm = 0,
-         int stale_window = 0, double stale_thr = 0.0) {
+         long long maxiter, uint32_t k_used, Ctl* ctl, double* partials, unsigned* counter, const int* nonfinite,
+         int warm = 0, int stale_window = 0, double stale_thr = 0.0) {
     pdl_wait();
     pdl_launch_dependents();
     constexpr int W = fl_w<K>(), P = fl_per_row<K>();
@@ -1305,6 +1305,9 @@ k_norm_b(uint32_t n, const double* __restrict__ b, const double* bmax, ColState*
         if ((uint32_t)k >= k_used) {
             s.done = 1;
             s.stop = STOP_ZERO_RHS;
+        } else if (*nonfinite) {   // rejected by the host once the solve is over: nothing to iterate on
+            s.done = 1;
+            s.stop = STOP_NONE;
         } else if (warm && !isfinite(beta)) {
             s.done = 1;
             s.err = ERR_WARM_NONFINITE;
@@ -1545,12 +1548,19 @@ __global__ void k_init_vectors(uint32_t n, double* __restrict__ v, double* __res
     }
 }
 
-// interleaved (internal order) -> column-major caller order
+// interleaved (internal order) -> column-major caller order; nothing is
+// written when the solve ends in an error (bad: non-finite input, ctl: a
+// device error), which the host reads after these
+__device__ __forceinline__ bool store_off(const int* bad, const Ctl* ctl) {
+    return (bad && *bad) || (ctl && ctl->err);
+}
 template <int K>
 __global__ void k_store_obs(uint32_t n, uint32_t k_used, const double* __restrict__ src,
-                            const uint32_t* __restrict__ perm, double* __restrict__ dst) {
+                            const uint32_t* __restrict__ perm, double* __restrict__ dst, const int* bad,
+                            const Ctl* ctl) {
     pdl_wait();
     pdl_launch_dependents();
+    if (store_off(bad, ctl)) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t d = perm ? perm[i] : i;
         double v[K];
@@ -1562,9 +1572,10 @@ __global__ void k_store_obs(uint32_t n, uint32_t k_used, const double* __restric
 }
 template <int K>
 __global__ void k_store_dofs(uint32_t n, uint32_t k_used, const double* __restrict__ src,
-                             double* __restrict__ dst) {
+                             double* __restrict__ dst, const int* bad, const Ctl* ctl) {
     pdl_wait();
     pdl_launch_dependents();
+    if (store_off(bad, ctl)) return;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         double v[K];
         ldk<K, double>(src + (size_t)j * K, v);
