@@ -100,9 +100,10 @@ struct RwParams {
 // Shared memory of the histogram terms: per-lane bins (bytes of all warps'
 // bins, 16-byte aligned) followed by one FP64 sum per bucket and warp; or
 // per-warp FP64 bins plus a 32 x K staging row per warp.
-template <int BIN_BYTES>
+// BL: bins per bucket and warp (32: one per lane).
+template <int BIN_BYTES, int BL = 32>
 __host__ __device__ constexpr size_t rw_private_bytes(int nb) {
-    return ((size_t)RW_WARPS * nb * 32 * BIN_BYTES + 15) / 16 * 16;
+    return ((size_t)RW_WARPS * nb * BL * BIN_BYTES + 15) / 16 * 16;
 }
 constexpr size_t RW_PRIVATE_LIMIT = 100 * 1024;   // 2 blocks per SM
 // dynamic shared memory any launch can ask for: the per-lane limit, or the
@@ -237,7 +238,7 @@ __device__ __forceinline__ double rw_load(const OpParamsT<T>& p, int t, int c, u
 // Block partials of ||u||^2 (modes 1, 3) and of the histogram bins in warp
 // order, then in the last block to finish: grand totals in block order and
 // the bins into A^T u (the runs that cross range boundaries: k_rw_fix).
-template <int K, int MODE, class T, bool SIMPLE>
+template <int K, int MODE, class T, bool SIMPLE, int BL = 32>
 __device__ __forceinline__ void rw_finish(const OpParamsT<T>& p, const RwParams& rw, const double (&accn)[K],
                                           const bool (&act)[K], ColState* cur, double* sq_out, int sq_stride) {
     using TO = std::conditional_t<MODE == 2, T, double>;
@@ -248,16 +249,16 @@ __device__ __forceinline__ void rw_finish(const OpParamsT<T>& p, const RwParams&
     __shared__ int is_last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nb = rw.n_buckets * K;
-    const BinT* pbins = reinterpret_cast<const BinT*>(rw_sm) + (size_t)wid * nb * 32;
+    const BinT* pbins = reinterpret_cast<const BinT*>(rw_sm) + (size_t)wid * nb * BL;
     double* wsums = reinterpret_cast<double*>(reinterpret_cast<char*>(rw_sm) +
-                                              rw_private_bytes<sizeof(BinT)>(nb)) + (size_t)wid * nb;
+                                              rw_private_bytes<sizeof(BinT), BL>(nb)) + (size_t)wid * nb;
     TO* atu = reinterpret_cast<TO*>(rw.atu);
     const int stride = K + nb;
     if (rw.hist_private) {   // lanes of each warp in order
         __syncwarp();
         for (int i = lane; i < nb; i += 32) {
             double s = 0.0;
-            for (int l = 0; l < 32; ++l) s += (double)pbins[i * 32 + l];
+            for (int l = 0; l < BL; ++l) s += (double)pbins[i * BL + l];
             wsums[i] = s;
         }
     }
@@ -277,7 +278,7 @@ __device__ __forceinline__ void rw_finish(const OpParamsT<T>& p, const RwParams&
     }
     {
         const double* base = rw.hist_private
-            ? reinterpret_cast<const double*>(reinterpret_cast<const char*>(rw_sm) + rw_private_bytes<sizeof(BinT)>(nb))
+            ? reinterpret_cast<const double*>(reinterpret_cast<const char*>(rw_sm) + rw_private_bytes<sizeof(BinT), BL>(nb))
             : rw_sm;
         for (int i = threadIdx.x; i < nb; i += RW_THREADS) {
             double s = 0.0;

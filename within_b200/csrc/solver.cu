@@ -1313,7 +1313,7 @@ TgKernel tg_kernel(int nq, bool wtd, bool demean) {
 }
 size_t tg_smem(int nq, bool wtd, bool demean) {
     const size_t stage = (size_t)TG_CH * (4 * nq + (demean ? 8 : 0) + (wtd && !demean ? 8 : 0));
-    return (size_t)RW_WARPS * TS_STAGES * (stage + sizeof(uint64_t));
+    return (size_t)RW_WARPS * TG_STAGES * (stage + sizeof(uint64_t));
 }
 // whether the staged gather applies to this solver's design (WITHIN_TSWEEP=0: never)
 bool tg_applies(const within_solver& s) {
@@ -1452,7 +1452,9 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
                 if (cls[t] == CLS_REST) rk.ts_slots.term[k++] = t;
         }
     }
-    rk.grid = rk.ts ? TS_GRID : rw_grid<K>();
+    // the staged sweep: as many blocks per SM as its bins and rings leave room for
+    rk.grid = !rk.ts ? rw_grid<K>()
+                     : 148 * (rk.ts_ns == 0 && rk.ts_smem <= TS_SMEM_FULL ? TS_BLOCKS_PER_SM : 2);
     uint64_t G = (uint64_t)rk.grid * RW_WARPS;   // ranges
     uint64_t CH = rw_chunk<K>(), min_range = CH;
     // several columns of an intercept-only design of at most three terms: the

@@ -31,9 +31,15 @@
 
 namespace wgpu {
 
-constexpr int TS_STAGES = 3;
-constexpr int TS_BLOCKS_PER_SM = 2;
-constexpr int TS_GRID = 148 * TS_BLOCKS_PER_SM;
+// The sweep is bound by latency and issue, not by its streams, so warps per SM
+// count: three blocks of 80 registers with two chunks in flight per warp took
+// 108 us for the LSMR step of the 10,000,000-row panel and 91 us for the adjoint,
+// two blocks with three chunks 122 and 103 us (130 and 97 with a bin per lane).
+constexpr int TS_STAGES = 2;
+constexpr int TS_BLOCKS_PER_SM = 3;
+// bins per bucket and warp: lanes l and l + 16 share one, the upper half adding
+// after the lower
+constexpr int TS_BIN_LANES = 16;
 constexpr int TS_MAXQ = 3;
 
 // Bytes of one chunk buffer: codes of NQ terms, u (K columns), sqrt(w).
@@ -47,7 +53,7 @@ __host__ __device__ constexpr uint32_t ts_chunk_bytes(int nq, bool weighted) {
 template <int K>
 __host__ __device__ constexpr size_t ts_hist_bytes(int n_buckets, int n_hist) {
     return n_hist == 0 ? 0
-                       : rw_private_bytes<8>(n_buckets * K) + (size_t)RW_WARPS * n_buckets * K * sizeof(double);
+                       : rw_private_bytes<8, TS_BIN_LANES>(n_buckets * K) + (size_t)RW_WARPS * n_buckets * K * sizeof(double);
 }
 template <int K>
 __host__ __device__ constexpr size_t ts_ring_offset(int n_buckets, int n_hist) {
@@ -58,7 +64,8 @@ __host__ __device__ constexpr size_t ts_smem_bytes(int n_buckets, int n_hist, in
     return ts_ring_offset<K>(n_buckets, n_hist) + (size_t)RW_WARPS * TS_STAGES * ts_chunk_bytes<K>(nq, weighted) +
            (size_t)RW_WARPS * TS_STAGES * sizeof(uint64_t);
 }
-constexpr size_t TS_SMEM_CAP = 112 * 1024;   // two blocks per SM
+constexpr size_t TS_SMEM_CAP = 112 * 1024;    // two blocks per SM
+constexpr size_t TS_SMEM_FULL = 74 * 1024;    // TS_BLOCKS_PER_SM blocks
 
 struct TsSlots {
     int term[TS_MAXQ];   // slot -> term: the run terms (rw.run order), then the hist terms, then the rest
@@ -104,7 +111,7 @@ __device__ __forceinline__ double ts_load(bool slope, const double (&sl)[R], int
 // 38 us, adjoint 57 -> 32 us against the generic sweep, whose loops over terms and
 // columns are not unrolled and which reads the slope again for every use.
 template <int K, int MODE, int NQ, int NRUN, int NHIST, bool WTD, int NS = 0>
-__global__ void __launch_bounds__(RW_THREADS, TS_BLOCKS_PER_SM)
+__global__ void __launch_bounds__(RW_THREADS, NS ? 2 : TS_BLOCKS_PER_SM)
 k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, double* __restrict__ u,
          ColState* cur, Ctl* ctl, int* err) {
     pdl_wait();
@@ -123,9 +130,10 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int nb = rw.n_buckets * K;
-    double* pbins = rw_sm + (size_t)wid * nb * 32;
+    double* pbins = rw_sm + (size_t)wid * nb * TS_BIN_LANES;
     if (NHIST > 0)
-        for (int i = lane; i < nb * 32; i += 32) pbins[i] = 0.0;
+        for (int i = lane; i < nb * TS_BIN_LANES; i += 32) pbins[i] = 0.0;
+    __syncwarp();
     char* ring = reinterpret_cast<char*>(rw_sm) + ts_ring_offset<K>(rw.n_buckets, NHIST) +
                  (size_t)wid * TS_STAGES * RG::STAGE_B;
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<char*>(rw_sm) +
@@ -357,35 +365,41 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
             }
         }
 
-        // ---- hist terms: per-lane bins, each lane adds its rows in order
+        // ---- hist terms: each lane adds its rows in order, the upper half warp after the lower
 #pragma unroll
-        for (int h = 0; h < NHIST; ++h) {
-            const int t = st_hist[h];
-            const int b0 = rw.hist[h].bucket0;
+        for (int half = 0; half < (NHIST > 0 ? 2 : 0); ++half) {
+            if ((lane >> 4) == half) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (r >= nr) continue;
-                uint32_t c = cd[0][r];
+                for (int h = 0; h < NHIST; ++h) {
+                    const int t = st_hist[h];
+                    const int b0 = rw.hist[h].bucket0;
 #pragma unroll
-                for (int q = 1; q < NQ; ++q)
-                    if (t == q) c = cd[q][r];
+                    for (int r = 0; r < R; ++r) {
+                        if (r >= nr) continue;
+                        uint32_t c = cd[0][r];
 #pragma unroll
-                for (int cc = 0; cc < MC; ++cc) {
-                    int nc = ncol[0];
-                    bool sc = slope[0][cc];
+                        for (int q = 1; q < NQ; ++q)
+                            if (t == q) c = cd[q][r];
 #pragma unroll
-                    for (int q = 1; q < NQ; ++q)
-                        if (t == q) {
-                            nc = ncol[q];
-                            sc = slope[q][cc];
+                        for (int cc = 0; cc < MC; ++cc) {
+                            int nc = ncol[0];
+                            bool sc = slope[0][cc];
+#pragma unroll
+                            for (int q = 1; q < NQ; ++q)
+                                if (t == q) {
+                                    nc = ncol[q];
+                                    sc = slope[q][cc];
+                                }
+                            if (cc >= nc) break;
+                            const int bk = b0 + (int)c * nc + cc;
+#pragma unroll
+                            for (int k = 0; k < K; ++k)
+                                pbins[(bk * K + k) * TS_BIN_LANES + (lane & 15)] += NS ? ts_load<R>(sc, sl, r) * b[r][k] : b[r][k];
                         }
-                    if (cc >= nc) break;
-                    const int bk = b0 + (int)c * nc + cc;
-#pragma unroll
-                    for (int k = 0; k < K; ++k)
-                        pbins[(bk * K + k) * 32 + lane] += NS ? ts_load<R>(sc, sl, r) * b[r][k] : b[r][k];
+                    }
                 }
             }
+            __syncwarp();
         }
 
         // ---- run terms
@@ -564,7 +578,7 @@ k_tsweep(OpParams p, RwParams rw, TsSlots sl, const double* __restrict__ v, doub
         }
     }
 
-    rw_finish<K, MODE, double, NS == 0>(p, rw, accn, act, cur, nullptr, 0);
+    rw_finish<K, MODE, double, NS == 0, TS_BIN_LANES>(p, rw, accn, act, cur, nullptr, 0);
 }
 
 }  // namespace wgpu
@@ -576,8 +590,9 @@ namespace wgpu {
 // demeaning out = yint - D x (solver.rs:468-473) for intercept-only designs
 // of at most three terms, one column: every warp walks chunks of 128 rows
 // (chunk w, w + warps, ...), its codes (and yint, sqrt(w)) brought into a
-// per-warp shared-memory ring by bulk copies TS_STAGES - 1 chunks ahead; the
+// per-warp shared-memory ring by bulk copies TG_STAGES - 1 chunks ahead; the
 // terms are summed in term order as in k_apply / k_demean (same bits).
+constexpr int TG_STAGES = 3;
 constexpr int TG_BLOCKS_PER_SM = 3;
 constexpr int TG_GRID = 148 * TG_BLOCKS_PER_SM;
 constexpr int TG_CH = 128;
@@ -591,7 +606,7 @@ struct TgRing {
 };
 template <int NQ, bool WTD, bool DEMEAN>
 __host__ __device__ constexpr size_t tg_smem_bytes() {
-    return (size_t)RW_WARPS * TS_STAGES * (TgRing<NQ, WTD, DEMEAN>::STAGE_B + sizeof(uint64_t));
+    return (size_t)RW_WARPS * TG_STAGES * (TgRing<NQ, WTD, DEMEAN>::STAGE_B + sizeof(uint64_t));
 }
 
 template <int NQ, bool WTD, bool DEMEAN>
@@ -618,9 +633,9 @@ k_tgather(OpParams p, const double* __restrict__ x, const double* __restrict__ y
     if (skip && *skip) return;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    char* ring = reinterpret_cast<char*>(tg_sm) + (size_t)wid * TS_STAGES * RG::STAGE_B;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(tg_sm + (size_t)RW_WARPS * TS_STAGES * RG::STAGE_B) +
-                     wid * TS_STAGES;
+    char* ring = reinterpret_cast<char*>(tg_sm) + (size_t)wid * TG_STAGES * RG::STAGE_B;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tg_sm + (size_t)RW_WARPS * TG_STAGES * RG::STAGE_B) +
+                     wid * TG_STAGES;
     const uint32_t warps = gridDim.x * RW_WARPS;
     const uint32_t w0 = blockIdx.x * RW_WARPS + wid;
     const uint32_t n_total = (p.n + TG_CH - 1) / TG_CH;
@@ -628,18 +643,18 @@ k_tgather(OpParams p, const double* __restrict__ x, const double* __restrict__ y
     auto chunk0 = [&](uint32_t j) -> uint32_t { return (w0 + j * warps) * TG_CH; };
     auto bulk_rows = [&](uint32_t j) -> uint32_t { return min((uint32_t)TG_CH, p.n - chunk0(j)) & ~3u; };
     if (lane == 0) {
-        for (int s = 0; s < TS_STAGES; ++s) mbar_init(&bars[s], 1);
+        for (int s = 0; s < TG_STAGES; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
     }
     __syncwarp();
     if (lane == 0)
-        for (uint32_t j = 0; j < (uint32_t)TS_STAGES && j < n_mine; ++j)
+        for (uint32_t j = 0; j < (uint32_t)TG_STAGES && j < n_mine; ++j)
             tg_issue<NQ, WTD, DEMEAN>(ring + j * RG::STAGE_B, &bars[j], p, yint, chunk0(j), bulk_rows(j));
     bool failed = false;
     uint32_t failed_at = 0;
     for (uint32_t j = 0; j < n_mine; ++j) {
-        const int stg = (int)(j % TS_STAGES);
-        const bool landed = mbar_wait_bounded(&bars[stg], (j / TS_STAGES) & 1u);
+        const int stg = (int)(j % TG_STAGES);
+        const bool landed = mbar_wait_bounded(&bars[stg], (j / TG_STAGES) & 1u);
         if (!__all_sync(FULL, landed)) {
             failed = true;
             failed_at = j;
@@ -688,10 +703,10 @@ k_tgather(OpParams p, const double* __restrict__ x, const double* __restrict__ y
             }
         }
         __syncwarp();
-        if (lane == 0 && j + TS_STAGES < n_mine) {
+        if (lane == 0 && j + TG_STAGES < n_mine) {
             fence_proxy_async_smem();
-            tg_issue<NQ, WTD, DEMEAN>(ring + stg * RG::STAGE_B, &bars[stg], p, yint, chunk0(j + TS_STAGES),
-                                      bulk_rows(j + TS_STAGES));
+            tg_issue<NQ, WTD, DEMEAN>(ring + stg * RG::STAGE_B, &bars[stg], p, yint, chunk0(j + TG_STAGES),
+                                      bulk_rows(j + TG_STAGES));
         }
         double s[R];
 #pragma unroll
@@ -716,8 +731,8 @@ k_tgather(OpParams p, const double* __restrict__ x, const double* __restrict__ y
     }
     if (failed) {
         if (lane == 0) atomicExch(err, ERR_WAIT_TIMEOUT);
-        for (uint32_t jj = failed_at; jj < n_mine && jj < failed_at + TS_STAGES; ++jj)
-            (void)mbar_wait_bounded(&bars[jj % TS_STAGES], (jj / TS_STAGES) & 1u);
+        for (uint32_t jj = failed_at; jj < n_mine && jj < failed_at + TG_STAGES; ++jj)
+            (void)mbar_wait_bounded(&bars[jj % TG_STAGES], (jj / TG_STAGES) & 1u);
     }
 }
 
