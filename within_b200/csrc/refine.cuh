@@ -108,14 +108,14 @@ k_cg_init(uint32_t n, const T* __restrict__ res, const T* __restrict__ z, T* __r
     double acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        T zv[K], rv[K];   // rows by 16-byte accesses, here and below
+        ldk<K, T>(z + (size_t)j * K, zv);
+        ldk<K, T>(res + (size_t)j * K, rv);
+        stk<K, T>(p + (size_t)j * K, zv);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const size_t o = (size_t)j * K + k;
-            const T zv = z[o];
-            p[o] = zv;
-            acc[k] += (double)res[o] * (double)zv;
-        }
+        for (int k = 0; k < K; ++k) acc[k] += (double)rv[k] * (double)zv[k];
+    }
     double tot[K];
     if (!grid_reduce<K>(acc, partials, counter, tot) || threadIdx.x != 0) return;
     if (first < 0) first = ctl->outer == 0 ? 1 : 0;
@@ -182,9 +182,13 @@ k_cg_alpha(uint32_t n, const T* __restrict__ p, const T* __restrict__ q, CgCol* 
     double acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        T pv[K], qv[K];
+        ldk<K, T>(p + (size_t)j * K, pv);
+        ldk<K, T>(q + (size_t)j * K, qv);
 #pragma unroll
-        for (int k = 0; k < K; ++k) acc[k] += (double)p[(size_t)j * K + k] * (double)q[(size_t)j * K + k];
+        for (int k = 0; k < K; ++k) acc[k] += (double)pv[k] * (double)qv[k];
+    }
     double tot[K];
     if (!grid_reduce<K>(acc, partials, counter, tot) || threadIdx.x != 0) return;
     for (int k = 0; k < K; ++k) {
@@ -213,14 +217,22 @@ __global__ void k_cg_update(uint32_t n, const T* __restrict__ p, const T* __rest
         act[k] = st[k].active != 0;
         a[k] = st[k].alpha;
     }
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const size_t o = (size_t)j * K;
+        T pv[K], qv[K], dv[K], rv[K];
+        ldk<K, T>(p + o, pv);
+        ldk<K, T>(q + o, qv);
+        ldk<K, T>(d + o, dv);
+        ldk<K, T>(res + o, rv);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            if (!act[k]) continue;
-            const size_t o = (size_t)j * K + k;
-            d[o] = (T)((double)d[o] + a[k] * (double)p[o]);
-            res[o] = (T)((double)res[o] - a[k] * (double)q[o]);
+            if (!act[k]) continue;   // a finished column keeps its values
+            dv[k] = (T)((double)dv[k] + a[k] * (double)pv[k]);
+            rv[k] = (T)((double)rv[k] - a[k] * (double)qv[k]);
         }
+        stk<K, T>(d + o, dv);
+        stk<K, T>(res + o, rv);
+    }
 }
 
 // rho' = <res, z>, beta = rho' / rho, the norm estimates and the stopping tests
@@ -234,9 +246,13 @@ k_cg_beta(uint32_t n, const T* __restrict__ res, const T* __restrict__ z, CgCol*
     double acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        T rv[K], zv[K];
+        ldk<K, T>(res + (size_t)j * K, rv);
+        ldk<K, T>(z + (size_t)j * K, zv);
 #pragma unroll
-        for (int k = 0; k < K; ++k) acc[k] += (double)res[(size_t)j * K + k] * (double)z[(size_t)j * K + k];
+        for (int k = 0; k < K; ++k) acc[k] += (double)rv[k] * (double)zv[k];
+    }
     double tot[K];
     if (!grid_reduce<K>(acc, partials, counter, tot) || threadIdx.x != 0) return;
     bool any = false;
@@ -280,13 +296,16 @@ __global__ void k_cg_dir(uint32_t n, const T* __restrict__ z, T* __restrict__ p,
         act[k] = st[k].active != 0;
         b[k] = st[k].beta;
     }
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const size_t o = (size_t)j * K;
+        T zv[K], pv[K];
+        ldk<K, T>(z + o, zv);
+        ldk<K, T>(p + o, pv);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (!act[k]) continue;
-            const size_t o = (size_t)j * K + k;
-            p[o] = (T)((double)z[o] + b[k] * (double)p[o]);
-        }
+        for (int k = 0; k < K; ++k)
+            if (act[k]) pv[k] = (T)((double)zv[k] + b[k] * (double)pv[k]);
+        stk<K, T>(p + o, pv);
+    }
 }
 
 // x += d (FP64 accumulation of the FP32 correction)

@@ -2139,11 +2139,11 @@ void cg_iteration(within_solver& s, within_solver::Work& w, within_solver::Mixed
         ++g_launches;
         scatter<K, 0, float>(s, m.t, m.q, nullptr, skip, st);
     }
-    launch_k(k_cg_alpha<K, float>, RED_GRID, RED_THREADS, 0, st, nd, m.p, m.q, m.st, m.ctl, w.partials, w.counter);
+    launch_k(k_cg_alpha<K, float>, grid_for(nd, RED_THREADS * 4, 148 * 4), RED_THREADS, 0, st, nd, m.p, m.q, m.st, m.ctl, w.partials, w.counter);
     launch_k(k_cg_update<K, float>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, m.p, m.q, m.d, m.res, m.st, m.ctl);
     g_launches += 2;
     precond_apply<K, float>(s, m.ctl, m.res, m.z, skip, st);
-    launch_k(k_cg_beta<K, float>, RED_GRID, RED_THREADS, 0, st, nd, m.res, m.z, m.st, m.ctl, w.partials, w.counter);
+    launch_k(k_cg_beta<K, float>, grid_for(nd, RED_THREADS * 4, 148 * 4), RED_THREADS, 0, st, nd, m.res, m.z, m.st, m.ctl, w.partials, w.counter);
     launch_k(k_cg_dir<K, float>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, m.z, m.p, m.st, m.ctl);
     g_launches += 2;
 }
@@ -2197,7 +2197,7 @@ void mixed_pre(within_solver& s, within_solver::Work& w, within_solver::MixedWor
     }
     launch_k(k_cg_start<K, float>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, m.g64, m.res, m.d);
     precond_apply<K, float>(s, m.ctl, m.res, m.z, nullptr, st);
-    launch_k(k_cg_init<K, float>, RED_GRID, RED_THREADS, 0, st, nd, m.res, m.z, m.p, m.st, m.ctl, first, w.partials,
+    launch_k(k_cg_init<K, float>, grid_for(nd, RED_THREADS * 4, 148 * 4), RED_THREADS, 0, st, nd, m.res, m.z, m.p, m.st, m.ctl, first, w.partials,
                                                            w.counter, use_h, h_in);
     g_launches += 2;
 }
