@@ -23,8 +23,8 @@
 //
 // 10,000,000-row panel, one column, against the scan engines: C^T 80 -> 49 us,
 // restrict 26 -> 15, means 22 -> 12.5, kept sums 11 -> 6, the run combine 25 ->
-// 21; eight columns: C^T 498 -> 128 us, restrict 148 -> 71, means 114 -> 44, run
-// combine 138 -> 53.  With four loads per lane requested at once C^T took 64 us
+// 21; eight columns: C^T 498 -> 116 us, restrict 148 -> 52, means 114 -> 44, run
+// combine 138 -> 51.  With four loads per lane requested at once C^T took 64 us
 // and eight-column restrict 150 us (there mostly the one warp that added the
 // 1700 partials of a segment cut for warps, hence pieces for blocks).
 #pragma once
@@ -45,9 +45,9 @@ constexpr int SL_BATCH = 8;
 // the medium segments (one warp each), then the short ones
 struct SLDev {
     const uint32_t* ptr;          // segment pointers
-    const uint32_t* short_ids;    // nullptr: short segment i is first + i
+    const uint32_t* short_ids;
     const uint32_t* medium_ids;
-    uint32_t first, n_short, n_medium, n_piece, medium_blocks;
+    uint32_t n_short, n_medium, n_piece, medium_blocks;
     const SLPiece* pieces;        // of this problem
     uint32_t piece_lo;            // its first piece's id
     const SLSplit* splits;
@@ -61,31 +61,52 @@ struct SLDev {
 //   V value(const Ctx&, uint32_t pos, const Idx&, int c0, bool valid) const;
 //   struct Pre; Pre pre(uint32_t seg, int c0) const;   what emit reads
 //   void emit(uint32_t seg, int c0, const Pre&, const V& s) const;
-template <class F, int K, int NB>
+// PF: the next batch's indices are requested before this batch's operands.
+template <class F, int K, int NB, bool PF>
 __device__ __forceinline__ FlVec<fl_w<K>()> sl_sum(const F& f, const typename F::Ctx& cx, uint32_t a, uint32_t b,
                                                    uint32_t stride, int c0) {
     constexpr int W = fl_w<K>();
     FlVec<W> s;
 #pragma unroll
     for (int i = 0; i < W; ++i) s.q[i] = 0.0;
-    for (uint32_t q = a; q < b; q += NB * stride) {
+    if constexpr (PF) {
+        if (a >= b) return s;
         typename F::Idx ix[NB];
 #pragma unroll
-        for (int j = 0; j < NB; ++j) ix[j] = f.index(min(q + j * stride, b - 1));
-        FlVec<W> v[NB];
+        for (int j = 0; j < NB; ++j) ix[j] = f.index(min(a + j * stride, b - 1));
+        for (uint32_t q = a; q < b; q += NB * stride) {
+            typename F::Idx nx[NB];   // the next batch's indices, requested before this one's operands
 #pragma unroll
-        for (int j = 0; j < NB; ++j) v[j] = f.value(cx, min(q + j * stride, b - 1), ix[j], c0, q + j * stride < b);
+            for (int j = 0; j < NB; ++j) nx[j] = f.index(min(q + (NB + j) * stride, b - 1));
+            FlVec<W> v[NB];
 #pragma unroll
-        for (int j = 0; j < NB; ++j)
+            for (int j = 0; j < NB; ++j) v[j] = f.value(cx, min(q + j * stride, b - 1), ix[j], c0, q + j * stride < b);
 #pragma unroll
-            for (int i = 0; i < W; ++i) s.q[i] += q + j * stride < b ? v[j].q[i] : 0.0;
+            for (int j = 0; j < NB; ++j)
+#pragma unroll
+                for (int i = 0; i < W; ++i) s.q[i] += q + j * stride < b ? v[j].q[i] : 0.0;
+#pragma unroll
+            for (int j = 0; j < NB; ++j) ix[j] = nx[j];
+        }
+    } else {
+        for (uint32_t q = a; q < b; q += NB * stride) {
+            typename F::Idx ix[NB];
+#pragma unroll
+            for (int j = 0; j < NB; ++j) ix[j] = f.index(min(q + j * stride, b - 1));
+            FlVec<W> v[NB];
+#pragma unroll
+            for (int j = 0; j < NB; ++j) v[j] = f.value(cx, min(q + j * stride, b - 1), ix[j], c0, q + j * stride < b);
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+#pragma unroll
+                for (int i = 0; i < W; ++i) s.q[i] += q + j * stride < b ? v[j].q[i] : 0.0;
+        }
     }
     return s;
 }
 
 template <class F, int K>
-__global__ void __launch_bounds__(SL_THREADS)
-k_seglist(F f, SLDev L, const int* __restrict__ skip) {
+__device__ __forceinline__ void seglist_body(const F& f, const SLDev& L, const int* __restrict__ skip) {
     pdl_wait();
     pdl_launch_dependents();
     constexpr int W = fl_w<K>(), P = fl_per_row<K>(), S = 32 / P;
@@ -103,10 +124,10 @@ k_seglist(F f, SLDev L, const int* __restrict__ skip) {
         const uint32_t t = (blockIdx.x - L.n_piece - L.medium_blocks) * SL_THREADS + threadIdx.x;
         const uint32_t i = t / P;
         if (i >= L.n_short) return;
-        const uint32_t seg = L.short_ids ? __ldg(L.short_ids + i) : L.first + i;
+        const uint32_t seg = __ldg(L.short_ids + i);
         const uint32_t a = __ldg(L.ptr + seg), b = __ldg(L.ptr + seg + 1);
         const typename F::Pre pre = f.pre(seg, c0);
-        f.emit(seg, c0, pre, sl_sum<F, K, F::SHORT_BATCH>(f, f.ctx(seg), a, b, 1, c0));
+        f.emit(seg, c0, pre, sl_sum<F, K, F::BATCH, false>(f, f.ctx(seg), a, b, 1, c0));
         return;
     }
     if (blockIdx.x >= L.n_piece) {   // medium segments
@@ -115,7 +136,7 @@ k_seglist(F f, SLDev L, const int* __restrict__ skip) {
         const uint32_t seg = __ldg(L.medium_ids + i);
         const uint32_t a = __ldg(L.ptr + seg), b = __ldg(L.ptr + seg + 1);
         const typename F::Pre pre = f.pre(seg, c0);
-        FlVec<W> s = sl_sum<F, K, SL_BATCH>(f, f.ctx(seg), a + g, b, S, c0);
+        FlVec<W> s = sl_sum<F, K, F::BATCH, F::PREFETCH>(f, f.ctx(seg), a + g, b, S, c0);
         tree(s);
         if (lane < P) f.emit(seg, c0, pre, s);
         return;
@@ -123,7 +144,7 @@ k_seglist(F f, SLDev L, const int* __restrict__ skip) {
     __shared__ __align__(16) double sm[SL_WARPS][K];
     __shared__ int last;
     const SLPiece pc = L.pieces[blockIdx.x];
-    FlVec<W> s = sl_sum<F, K, SL_BATCH>(f, f.ctx(pc.seg), pc.p0 + wid * S + g, pc.p1, SL_WARPS * S, c0);
+    FlVec<W> s = sl_sum<F, K, F::BATCH, F::PREFETCH>(f, f.ctx(pc.seg), pc.p0 + wid * S + g, pc.p1, SL_WARPS * S, c0);
     tree(s);
     if (lane < P) fl_st<W>(&sm[wid][c0], s);
     __syncthreads();
@@ -162,52 +183,43 @@ k_seglist(F f, SLDev L, const int* __restrict__ skip) {
     }
 }
 
-// One column, every segment short: a warp's 32 segments are 32 consecutive runs
-// of positions, so the warp computes their values with coalesced reads into
-// shared memory and every lane then adds its own segment's in position order
-// (the sum of one lane reading them from memory, bit for bit).  C on the panel
-// (10.4 M non-zeros in rows of about ten): 70 -> 66 us.  More shared memory per
-// warp than 2 KB, or more than six blocks per SM, takes L1 from the gathered
-// operand: 116 us with 4 KB and six blocks, 127 us with eight.
-constexpr uint32_t SL_STAGE = 256;   // values staged per warp; wider groups read memory directly
+template <class F, int K>
+__global__ void __launch_bounds__(SL_THREADS)
+k_seglist(F f, SLDev L, const int* __restrict__ skip) {
+    seglist_body<F, K>(f, L, skip);
+}
+// the same held to 32 registers, eight blocks per SM (F::FULL)
+template <class F, int K>
+__global__ void __launch_bounds__(SL_THREADS, 8)
+k_seglist_full(F f, SLDev L, const int* __restrict__ skip) {
+    seglist_body<F, K>(f, L, skip);
+}
 
-template <class F>
-__global__ void __launch_bounds__(SL_THREADS, 6)
-k_segstage(F f, const uint32_t* __restrict__ ptr, uint32_t first, uint32_t n_seg, const int* __restrict__ skip) {
+// Every segment short (the rows of C, the prolongation, most rounds): one group
+// of lanes per segment, in position order.  Nothing but resident warps hides the
+// two or three dependent loads of so little work, so the kernel is held to 32
+// registers (eight blocks per SM) and asks for two positions at a time: C of the
+// 10,000,000-row panel (10.4 M non-zeros in rows of about five) takes 62 us with
+// one column and 146 us with eight; 236 us with eight positions at a time in 64
+// registers, 183 us with four in 40, 66 us (one column) with the values of a
+// warp's segments staged in shared memory.
+constexpr int SL_SHORT_BATCH = 2;
+
+template <class F, int K>
+__global__ void __launch_bounds__(SL_THREADS, 8)
+k_segshort(F f, const uint32_t* __restrict__ ptr, uint32_t first, uint32_t n_seg, const int* __restrict__ skip) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ double sm[SL_WARPS][SL_STAGE];
+    constexpr int W = fl_w<K>(), P = fl_per_row<K>();
     if (skip && *skip) return;
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t i0 = (blockIdx.x * SL_WARPS + wid) * 32u;
-    if (i0 >= n_seg) return;   // whole warps
-    const bool mine = i0 + lane < n_seg;
-    const uint32_t seg = first + (mine ? i0 + lane : n_seg - 1);
-    const uint32_t b = __ldg(ptr + seg + 1), a = mine ? __ldg(ptr + seg) : b;
-    const uint32_t w0 = __shfl_sync(FULL, a, 0), w1 = __shfl_sync(FULL, b, 31);
-    const typename F::Pre pre = f.pre(seg, 0);
-    const typename F::Ctx cx = f.ctx(seg);
-    FlVec<1> s;
-    if (w1 - w0 <= SL_STAGE) {
-        for (uint32_t q = w0 + lane; q < w1; q += SL_BATCH * 32) {
-            typename F::Idx ix[SL_BATCH];
-#pragma unroll
-            for (int j = 0; j < SL_BATCH; ++j) ix[j] = f.index(min(q + 32 * j, w1 - 1));
-            FlVec<1> v[SL_BATCH];
-#pragma unroll
-            for (int j = 0; j < SL_BATCH; ++j) v[j] = f.value(cx, min(q + 32 * j, w1 - 1), ix[j], 0, q + 32 * j < w1);
-#pragma unroll
-            for (int j = 0; j < SL_BATCH; ++j)
-                if (q + 32 * j < w1) sm[wid][q + 32 * j - w0] = v[j].q[0];
-        }
-        __syncwarp();
-        s.q[0] = 0.0;
-        for (uint32_t p = a; p < b; ++p) s.q[0] += sm[wid][p - w0];
-    } else {
-        s = sl_sum<F, 1, SL_BATCH>(f, cx, a, b, 1, 0);
-    }
-    if (mine) f.emit(seg, 0, pre, s);
+    const uint32_t t = blockIdx.x * SL_THREADS + threadIdx.x;
+    const uint32_t i = t / P;
+    const int c0 = (int)(t % P) * W;
+    if (i >= n_seg) return;
+    const uint32_t seg = first + i;
+    const uint32_t a = __ldg(ptr + seg), b = __ldg(ptr + seg + 1);
+    const typename F::Pre pre = f.pre(seg, c0);
+    f.emit(seg, c0, pre, sl_sum<F, K, SL_SHORT_BATCH, false>(f, f.ctx(seg), a, b, 1, c0));
 }
 
 // ---------------------------------------------------------------------------
@@ -215,8 +227,13 @@ k_segstage(F f, const uint32_t* __restrict__ ptr, uint32_t first, uint32_t n_seg
 // sums are those of the functors of the same name in kernels.cuh, FP64.
 template <int K>
 struct SlBase {
-    static constexpr bool STAGED = false;   // one column, short segments only: k_segstage
-    static constexpr int SHORT_BATCH = SL_BATCH;   // positions of a short segment a lane requests at once
+    // medium and long segments: positions a lane requests at once, whether the
+    // next batch's indices come before this batch's operands, and whether the
+    // kernel is held to eight blocks per SM.  With indices ahead C^T
+    // went from 126 to 116 us at eight columns and from 27 to 22 at four, the
+    // forward rounds from 40 to 17 and from 14 to 9.
+    static constexpr int BATCH = SL_BATCH;
+    static constexpr bool PREFETCH = true, FULL = false;
     static constexpr int W = fl_w<K>();
     using V = FlVec<W>;
     struct Ctx {};
@@ -277,6 +294,10 @@ struct SlBase {
 
 template <int K>
 struct SlRestrict : SlBase<K> {
+    // it streams: resident warps are worth more than loads per lane (71 -> 52 us at
+    // eight columns, 14 -> 10 at four)
+    static constexpr int BATCH = 4;
+    static constexpr bool PREFETCH = false, FULL = true;
     SL_TYPES;
     using Ctx = typename B::Ctx;
     using Pre = typename B::MeanPre;
@@ -432,7 +453,6 @@ struct SlBwd : SlBase<K> {
 
 template <int K>
 struct SlC : SlBase<K> {
-    static constexpr bool STAGED = true;
     SL_TYPES;
     using Ctx = typename B::Ctx;
     struct Pre {
@@ -464,6 +484,7 @@ struct SlC : SlBase<K> {
 
 template <int K>
 struct SlMean : SlBase<K> {
+    static constexpr bool PREFETCH = false;
     SL_TYPES;
     using Pre = typename B::MeanPre;
     struct Ctx {
@@ -487,7 +508,6 @@ struct SlMean : SlBase<K> {
 
 template <int K>
 struct SlProlong : SlBase<K> {
-    static constexpr int SHORT_BATCH = 2;   // a level lies in as many subdomains as its term has partners
     SL_TYPES;
     using Ctx = typename B::Ctx;
     struct Pre {};
@@ -684,8 +704,8 @@ k_rounds(SchwarzDev S, RDev R, uint32_t row_lo, uint32_t row_hi, uint32_t n_red,
 // of the term's level-sorted order
 template <int K>
 struct SlScatter {
-    static constexpr bool STAGED = false;
-    static constexpr int SHORT_BATCH = SL_BATCH;
+    static constexpr int BATCH = SL_BATCH;
+    static constexpr bool PREFETCH = true, FULL = false;
     static constexpr int W = fl_w<K>();
     using V = FlVec<W>;
     struct Ctx {};

@@ -374,20 +374,18 @@ constexpr uint32_t SL_TARGET_BLOCKS = 148 * 6;
 
 template <class F, int K>
 void launch_sl(const F& f, const DevBook& b, const SLPart& p, const uint32_t* ptr, const int* skip, cudaStream_t st) {
-    if constexpr (K == 1 && F::STAGED) {
-        if (p.all_short) {
-            if (!p.n_short) return;
-            launch_k(k_segstage<F>, (p.n_short + SL_THREADS - 1) / SL_THREADS, SL_THREADS, 0, st, f, ptr, p.first,
-                     p.n_short, skip);
-            ++g_launches;
-            return;
-        }
+    if (p.all_short) {
+        if (!p.n_short) return;
+        const uint64_t threads = (uint64_t)p.n_short * fl_per_row<K>();
+        launch_k(k_segshort<F, K>, (unsigned)((threads + SL_THREADS - 1) / SL_THREADS), SL_THREADS, 0, st, f, ptr,
+                 p.first, p.n_short, skip);
+        ++g_launches;
+        return;
     }
     SLDev L;
     L.ptr = ptr;
-    L.short_ids = p.all_short ? nullptr : b.short_ids + p.short_off;
+    L.short_ids = b.short_ids + p.short_off;
     L.medium_ids = b.medium_ids + p.medium_lo;
-    L.first = p.first;
     L.n_short = p.n_short;
     L.n_medium = p.medium_hi - p.medium_lo;
     L.n_piece = p.piece_hi - p.piece_lo;
@@ -400,7 +398,8 @@ void launch_sl(const F& f, const DevBook& b, const SLPart& p, const uint32_t* pt
     const uint32_t short_blocks = (uint32_t)(((uint64_t)p.n_short * fl_per_row<K>() + SL_THREADS - 1) / SL_THREADS);
     const uint32_t grid = L.n_piece + L.medium_blocks + short_blocks;
     if (!grid) return;
-    launch_k(k_seglist<F, K>, grid, SL_THREADS, 0, st, f, L, skip);
+    if constexpr (F::FULL) launch_k(k_seglist_full<F, K>, grid, SL_THREADS, 0, st, f, L, skip);
+    else launch_k(k_seglist<F, K>, grid, SL_THREADS, 0, st, f, L, skip);
     ++g_launches;
 }
 
