@@ -813,9 +813,15 @@ def _family(name):
         return "gather"
     if name.startswith("k_demean"):
         return "demean"
+    if name.startswith("k_csweep"):
+        mode = name.split(",")[1].strip()
+        return "sweep_lsmr" if mode == "1" else ("sweep_adjoint" if mode == "0" else None)
+    if name.startswith("k_rounds"):   # all narrow rounds of one direction
+        return "BwdF" if name.rstrip(">").rstrip().endswith("true") else "FwdF"
     for f in ("ScatterF", "CtF", "CF<", "FwdF", "BwdF", "DenseF", "CoreF", "RestrictF", "MeanF", "KeptSumF",
               "ProlongF"):
-        if f in name:
+        # the list engine's functors are named Sl<step><K>, the others' <step>F<K, type>
+        if f in name or "Sl" + f.rstrip("<")[:-1] + "<" in name:
             return f.rstrip("<")
     for k, f in (("k_ptilde", "ptilde"), ("k_alpha_step", "alpha"), ("k_solution_update", "solution_update")):
         if name.startswith(k):
