@@ -71,12 +71,11 @@ def parse():
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the
 # design-operator pair's kernels, from one ncu capture (--clock-control none)
 # of the 4,000,000-row panel: the staged gather k_tgather<3,0,0> (D x) and the
-# staged adjoint sweep k_tsweep<1,0,3,2,1,0> with its crossing-run fix-up
-# k_rw_fix<1,0> and the warp-range run combine segsweep_kernel<ScatterF<1,0>>
-# (D^T u).  Every stream of the pair grows with the row count on this panel
+# staged adjoint sweep k_tsweep<1,0,3,2,1,0,0> with its crossing-run fix-up
+# k_rw_fix<1,0> and the run combine k_seglist<SlScatter<1>> (D^T u).  Every stream of the pair grows with the row count on this panel
 # generator (workers n/10, firms n/100), so a 10,000,000-row launch moves 2.5x.
-PAIR_TRAFFIC_4M = {"gather": 51_800_064, "adjoint": 90_200_832}
-PAIR_TRAFFIC_KERNELS = "k_tgather<3,0,0> + k_tsweep<1,0,3,2,1,0> + k_rw_fix<1,0> + segsweep_kernel<ScatterF<1,0>>"
+PAIR_TRAFFIC_4M = {"gather": 51_707_904, "adjoint": 90_450_944}
+PAIR_TRAFFIC_KERNELS = "k_tgather<3,0,0> + k_tsweep<1,0,3,2,1,0,0> + k_rw_fix<1,0> + k_seglist<SlScatter<1>>"
 
 
 def pair_traffic(n, q, solver):
@@ -88,7 +87,7 @@ def pair_traffic(n, q, solver):
         ranges = int(os.environ.get("WITHIN_WARP_RANGES", "1"))
     else:
         staged, ranges = t.get("staged_sweep", 1) == 1, t.get("warp_ranges", 1)
-    if q != 3 or not staged or ranges < 1:
+    if q != 3 or not staged or ranges != 1:
         return None, None
     f = n / 4_000_000
     return (f * (PAIR_TRAFFIC_4M["gather"] + PAIR_TRAFFIC_4M["adjoint"]),
