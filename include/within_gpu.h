@@ -358,6 +358,15 @@ int within_demean_vjp(uint64_t n, uint64_t k, const double* r_dev, const double*
                       const double* s_dev, const double* w_dev, double* grad_z_dev,
                       double* grad_w_dev, void* stream);
 
+/* ---- Failure injection, for tests of a caller's error handling ----
+ * Leaves the error word that a timed-out device wait leaves (a four-byte copy;
+ * no kernel runs or waits).  The solver's next solve, or the preconditioner's
+ * next apply, then fails with WITHIN_ERR_CUDA without writing its outputs, and
+ * the one after it runs as usual.  A preconditioner whose apply has no kernel
+ * that waits never fails so. */
+int within_solver_inject_timeout(within_solver* s);
+int within_preconditioner_inject_timeout(within_preconditioner* p);
+
 /* ---- diagnostics ---- */
 const char* within_last_error(void);
 /* Kernel launches issued by this library on the calling thread since the last

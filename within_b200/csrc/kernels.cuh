@@ -916,6 +916,16 @@ __device__ __forceinline__ void givens(double a, double b, double& c, double& s,
     }
 }
 
+// Whether the device has raised an error in this solve; one that a wait outside
+// the solve's own word left (werr: the solver's) is taken over.  It ends every
+// column, so that no later kernel of the loop runs on vectors a failed one left
+// unwritten or waits out its own limit.  One thread.
+__device__ __forceinline__ int device_error(Ctl* ctl, const int* werr) {
+    const int e = *(const volatile int*)werr;
+    if (e) atomicCAS(&ctl->err, 0, e);
+    return *(volatile int*)&ctl->err != 0 ? 1 : 0;
+}
+
 // One column of k_alpha_step from its sums <v, p~>, <v, v> and <p~, p~>:
 // alpha with the indefinite-M check, the recurrences, the stopping tests.
 // Returns whether the column has finished.
@@ -1011,7 +1021,7 @@ __device__ __forceinline__ bool alpha_column(const ColState& cur, ColState* nxt,
 template <int K>
 __global__ void __launch_bounds__(RED_THREADS)
 k_alpha_step(uint32_t n, const double* __restrict__ v, const double* __restrict__ p,
-             const ColState* cur, ColState* nxt, Ctl* ctl, double* partials, unsigned* counter) {
+             const ColState* cur, ColState* nxt, Ctl* ctl, const int* werr, double* partials, unsigned* counter) {
     pdl_wait();
     pdl_launch_dependents();
     if (ctl->all_done) return;
@@ -1049,9 +1059,10 @@ k_alpha_step(uint32_t n, const double* __restrict__ v, const double* __restrict_
         int all = 1;
         for (int k = 0; k < K; ++k) all &= col_done[k];
         ctl->k5_skip = 0;
-        ctl->all_done = all;
+        ctl->all_done = all | device_error(ctl, werr);
     }
 }
+
 // v <- v / alpha; h_bar, x, h update (recurrence.rs:143-191)
 // Ring of the last `cap` (v, p/alpha) pairs for the windowed M-orthogonal
 // reorthogonalisation (bidiag.rs:113-217, 489-512); cap = 0 disables it.
@@ -1448,7 +1459,7 @@ __global__ void k_scale_u(uint32_t n, const double* __restrict__ b, double* __re
 template <int K>
 __global__ void __launch_bounds__(RED_THREADS)
 k_alpha_init(uint32_t n, const double* __restrict__ v, const double* __restrict__ p, ColState* st,
-             ColState* st_other, Ctl* ctl, double* partials, unsigned* counter) {
+             ColState* st_other, Ctl* ctl, const int* werr, double* partials, unsigned* counter) {
     pdl_wait();
     pdl_launch_dependents();
     constexpr int W = fl_w<K>(), P = fl_per_row<K>();
@@ -1507,7 +1518,7 @@ k_alpha_init(uint32_t n, const double* __restrict__ v, const double* __restrict_
         st_other[k] = s;
         all = all && s.done;
     }
-    ctl->all_done = all ? 1 : 0;
+    ctl->all_done = (all ? 1 : 0) | device_error(ctl, werr);
     ctl->k5_skip = 0;
 }
 
@@ -1550,17 +1561,18 @@ __global__ void k_init_vectors(uint32_t n, double* __restrict__ v, double* __res
 
 // interleaved (internal order) -> column-major caller order; nothing is
 // written when the solve ends in an error (bad: non-finite input, ctl: a
-// device error), which the host reads after these
-__device__ __forceinline__ bool store_off(const int* bad, const Ctl* ctl) {
-    return (bad && *bad) || (ctl && ctl->err);
+// device error, werr: a timed-out wait of the demeaning gather), which the host
+// reads after these
+__device__ __forceinline__ bool store_off(const int* bad, const Ctl* ctl, const int* werr) {
+    return (bad && *bad) || (ctl && ctl->err) || *werr;
 }
 template <int K>
 __global__ void k_store_obs(uint32_t n, uint32_t k_used, const double* __restrict__ src,
                             const uint32_t* __restrict__ perm, double* __restrict__ dst, const int* bad,
-                            const Ctl* ctl) {
+                            const Ctl* ctl, const int* werr) {
     pdl_wait();
     pdl_launch_dependents();
-    if (store_off(bad, ctl)) return;
+    if (store_off(bad, ctl, werr)) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t d = perm ? perm[i] : i;
         double v[K];
@@ -1572,10 +1584,10 @@ __global__ void k_store_obs(uint32_t n, uint32_t k_used, const double* __restric
 }
 template <int K>
 __global__ void k_store_dofs(uint32_t n, uint32_t k_used, const double* __restrict__ src,
-                             double* __restrict__ dst, const int* bad, const Ctl* ctl) {
+                             double* __restrict__ dst, const int* bad, const Ctl* ctl, const int* werr) {
     pdl_wait();
     pdl_launch_dependents();
-    if (store_off(bad, ctl)) return;
+    if (store_off(bad, ctl, werr)) return;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         double v[K];
         ldk<K, double>(src + (size_t)j * K, v);

@@ -585,7 +585,8 @@ k_rounds(SchwarzDev S, RDev R, uint32_t row_lo, uint32_t row_hi, uint32_t n_red,
         for (uint32_t i = 0; i < RP_STAGES; ++i) mbar_init(&bar[i], 1);
         fence_mbar_init();
     }
-    __syncthreads();
+    // an earlier wait has timed out: this launch's result is not used, and its waits would run out as well
+    if (__syncthreads_or(tid == 0 && *(const volatile int*)err != 0)) return;
     // the last warp's first lane has the passes copied (sizes are multiples of 16 bytes), the others sum
     const bool copies = tid == RP_THREADS;
     auto issue = [&](uint32_t p) {

@@ -917,9 +917,11 @@ SchwarzWorkT<float>& schwarz_user_work_f(SchwarzUser& U, const within_preconditi
     return kp.wf;
 }
 
+// skip: nothing runs when set.  keep (optional): z is left as it is when set by
+// the time the last kernel runs.
 template <int K, class T = double>
 void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, const int* skip,
-                   cudaStream_t st) {
+                   cudaStream_t st, const int* keep = nullptr) {
     KPlans& kp = schwarz_user_plans(U, P, K);
     SchwarzDevT<T> S;
     SchwarzWorkT<T>* w;
@@ -975,7 +977,7 @@ void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, c
             for (uint32_t q = L.narrow_lo; q-- > 0;) launch_sl<SlBwd<K>, K>({{S}}, b, L.bwd[q], P.bwd_ptr, skip, st);
             launch_sl<SlC<K>, K>({{S}}, b, L.c, P.c_ptr, skip, st);
             launch_sl<SlMean<K>, K>({{S}}, b, L.restrict_, S.loc_ptr, skip, st);
-            launch_sl<SlProlong<K>, K>({{S}, z}, b, L.prolong, P.dof_ptr, skip, st);
+            launch_sl<SlProlong<K>, K>({{S}, z}, b, L.prolong, P.dof_ptr, keep ? keep : skip, st);
             return;
         }
     }
@@ -1011,6 +1013,29 @@ void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, c
 }
 
 }  // namespace
+
+// A solver's (or standalone preconditioner's) error word: set by a kernel whose
+// wait timed out, reported and cleared by the call that reads it.
+constexpr const char* WAIT_TIMEOUT_TEXT = "a bulk copy into shared memory did not complete within 1 s";
+void clear_word(int* word, cudaStream_t st) {
+    CK(cudaMemsetAsync(word, 0, sizeof(int), st));
+    CK(cudaStreamSynchronize(st));
+}
+void raise_word(int* word) {
+    CK(cudaDeviceSynchronize());
+    const int e = ERR_WAIT_TIMEOUT;
+    CK(cudaMemcpy(word, &e, sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaDeviceSynchronize());
+}
+// waits for the stream
+void check_word(int* word, cudaStream_t st) {
+    int e = 0;
+    CK(cudaMemcpyAsync(&e, word, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (!e) return;
+    clear_word(word, st);
+    throw WError(ERR_CUDA, WAIT_TIMEOUT_TEXT);
+}
 
 // What the host reads when a solve is over.
 struct SolveState {
@@ -1862,7 +1887,8 @@ void iteration(within_solver& s, within_solver::Work& w, int par, cudaStream_t s
         launch_k(k_reorth_axpy<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, j, w.ring, w.v, w.p, cur, w.ctl, w.coef);
         g_launches += 2;
     }
-    launch_k(k_alpha_step<K>, fl_grid<K>(nd), RED_THREADS, 0, st, nd, w.v, w.p, cur, nxt, w.ctl, w.partials, w.counter);
+    launch_k(k_alpha_step<K>, fl_grid<K>(nd), RED_THREADS, 0, st, nd, w.v, w.p, cur, nxt, w.ctl, s.sweep_err, w.partials,
+             w.counter);
     ++g_launches;
     launch_k(k_solution_update<K>, fl_vec_grid<K>(nd), 256, 0, st, nd, w.v, w.h, w.hb, w.x, nxt, w.ctl, w.ring,
                                                                       w.p);
@@ -1931,7 +1957,8 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
               double t_setup0, const SolveExt& ext = SolveExt{}, int32_t* stop_out = nullptr) {
     const uint32_t n = (uint32_t)s.n_obs, nd = (uint32_t)s.n_dofs;
     // queued to the end without a host wait: a non-finite input or a device error
-    // ends every column at once and keeps the outputs from being written, and the
+    // (its own word, or the solver's set by a timed-out wait: device_error, store_off)
+    // ends every column and keeps the outputs from being written, and the
     // host reads it with the results (a wait here, one after the loop and two more
     // copies cost a solve of 2,003 rows 208 us instead of 162)
     CK(cudaMemsetAsync(w.ctl, 0, sizeof(SolveState) - offsetof(SolveState, ctl), st));
@@ -1964,8 +1991,8 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
         scatter<K, 0>(s, w.u, w.p, w.st, nullptr, st);
     }
     precond_apply<K>(s, w.ctl, w.p, w.v, nullptr, st);
-    launch_k(k_alpha_init<K>, fl_grid<K>(nd), RED_THREADS, 0, st, nd, w.v, w.p, w.st, w.st + 8, w.ctl, w.partials,
-                                                      w.counter);
+    launch_k(k_alpha_init<K>, fl_grid<K>(nd), RED_THREADS, 0, st, nd, w.v, w.p, w.st, w.st + 8, w.ctl, s.sweep_err,
+             w.partials, w.counter);
     launch_k(k_init_vectors<K>, fl_vec_grid<K>(nd), 256, 0, st, nd, w.v, w.h, w.hb, w.x, w.st, w.ring, w.p);
     g_launches += 6;
     const bool device_loop = build_loop_graph<K>(s, w);
@@ -2016,11 +2043,12 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
     }
     if (D_out) {
         launch_k(k_store_obs<K>, grid_for(n, 256, 148 * 16), 256, 0, st, n, k_used, w.dm, s.perm, D_out, w.nonfinite,
-                 w.ctl);
+                 w.ctl, s.sweep_err);
         ++g_launches;
     }
     if (X_out) {
-        launch_k(k_store_dofs<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, k_used, w.x, X_out, w.nonfinite, w.ctl);
+        launch_k(k_store_dofs<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, k_used, w.x, X_out, w.nonfinite, w.ctl,
+                 s.sweep_err);
         ++g_launches;
     }
     ColState fin[8];
@@ -2029,16 +2057,17 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
     CK(cudaMemcpyAsync(&out, w.state, sizeof(SolveState), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (device_loop) g_launches += (uint64_t)out.ctl.bodies_run * w.graph_iters;
+    if (out.sweep_err) clear_word(s.sweep_err, st);   // reported below: the next call starts clean
     if (out.nonfinite)
         throw WError(ERR_INVALID, ext.x0 ? "response and warm start must be finite (a non-finite value was found)"
                                          : "response must be finite (a non-finite value was found)");
     if (out.ctl.err == 5)
         throw WError(ERR_INDEFINITE, "mlsmr: preconditioner not positive definite (<v, Mv> < 0)");
     if (out.ctl.err == ERR_WAIT_TIMEOUT)
-        throw WError(ERR_CUDA, "row sweep: a bulk copy into shared memory did not complete within 1 s");
+        throw WError(ERR_CUDA, WAIT_TIMEOUT_TEXT);
     if (out.ctl.err == ERR_WARM_NONFINITE)
         throw WError(ERR_INVALID, "warm-start residual b - A x0 has a non-finite norm");
-    if (out.sweep_err) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
+    if (out.sweep_err) throw WError(ERR_CUDA, WAIT_TIMEOUT_TEXT);
     const double t_solve1 = now_s();
     // the state parity after the loop is whichever buffer was written last:
     // both buffers hold identical done states for finished columns, so read
@@ -2344,18 +2373,15 @@ void run_mixed(within_solver& s, const double* Y, uint32_t k_used, double tol, u
     }
     if (D_out) {
         launch_k(k_store_obs<K>, grid_for(n, 256, 148 * 16), 256, 0, st, n, k_used, w.dm, s.perm, D_out,
-                 (const int*)nullptr, (const Ctl*)nullptr);
+                 (const int*)nullptr, (const Ctl*)nullptr, s.sweep_err);
         ++g_launches;
     }
     if (X_out) {
         launch_k(k_store_dofs<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, k_used, m.x64, X_out, (const int*)nullptr,
-                 (const Ctl*)nullptr);
+                 (const Ctl*)nullptr, s.sweep_err);
         ++g_launches;
     }
-    int werr = 0;
-    CK(cudaMemcpyAsync(&werr, s.sweep_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (werr) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
+    check_word(s.sweep_err, st);
     const double t_end = now_s();
     if (stats)
         for (uint32_t k = 0; k < k_used; ++k) {
@@ -3244,12 +3270,7 @@ int within_solver_operator_apply(within_solver* s, const double* x_dev, double* 
             ++g_launches;
         }
         CK(cudaGetLastError());
-        if (!stream) {
-            CK(cudaStreamSynchronize(st));
-            int e = 0;
-            CK(cudaMemcpy(&e, s->sweep_err, sizeof(int), cudaMemcpyDeviceToHost));
-            if (e) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
-        }
+        if (!stream) check_word(s->sweep_err, st);
     });
 }
 
@@ -3267,12 +3288,7 @@ int within_solver_operator_apply_adjoint(within_solver* s, const double* u_dev, 
                                           nullptr, nullptr, 0, st);
             rowsweep_rest<1, double>(*s, rk, u_dev, y_dev, nullptr, st);
             CK(cudaGetLastError());
-            if (!stream) {
-                CK(cudaStreamSynchronize(st));
-                int e = 0;
-                CK(cudaMemcpy(&e, s->sweep_err, sizeof(int), cudaMemcpyDeviceToHost));
-                if (e) throw WError(ERR_CUDA, "row sweep: a bulk copy into shared memory did not complete within 1 s");
-            }
+            if (!stream) check_word(s->sweep_err, st);
             return;
         }
         scatter<1, 0>(*s, u_dev, y_dev, nullptr, nullptr, st);
@@ -3471,7 +3487,7 @@ int within_preconditioner_apply(const within_preconditioner* pc, const double* x
         auto* p = const_cast<within_preconditioner*>(pc);
         set_device(p->device);
         cudaStream_t st = stream ? (cudaStream_t)stream : nullptr;
-        int werr = 0;
+        int* werr = nullptr;
         if (p->kind == 2) {
             launch_k(k_diag_apply<1>, grid_for(p->n, 256, 148 * 8), 256, 0, st, p->n, p->inv_diag, x_dev, y_dev, nullptr);
             ++g_launches;
@@ -3481,13 +3497,29 @@ int within_preconditioner_apply(const within_preconditioner* pc, const double* x
                 p->standalone = new SchwarzUser();
                 p->standalone->tuning = resolve_tuning(nullptr);
             }
-            schwarz_apply<1>(*p, *p->standalone, x_dev, y_dev, nullptr, st);
-            if (p->standalone->lists.fwd_narrow.n_pass)
-                CK(cudaMemcpyAsync(&werr, p->standalone->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+            schwarz_user_plans(*p->standalone, *p, 1);
+            if (p->standalone->lists.fwd_narrow.n_pass) werr = p->standalone->err;   // else no kernel waits
+            schwarz_apply<1>(*p, *p->standalone, x_dev, y_dev, nullptr, st, werr);
         }
         CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(st));
-        if (werr) throw WError(ERR_CUDA, "a bulk copy into shared memory did not complete within 1 s");
+        if (werr) check_word(werr, st);
+        else CK(cudaStreamSynchronize(st));
+    });
+}
+
+int within_solver_inject_timeout(within_solver* s) {
+    return guarded([&] {
+        std::lock_guard<std::mutex> g(s->mu);
+        set_device(s->device);
+        raise_word(s->sweep_err);
+    });
+}
+int within_preconditioner_inject_timeout(within_preconditioner* p) {
+    return guarded([&] {
+        std::lock_guard<std::mutex> g(p->mu);
+        set_device(p->device);
+        if (!p->standalone || !p->standalone->err) throw WError(ERR_INVALID, "the preconditioner has not been applied yet");
+        raise_word(p->standalone->err);
     });
 }
 
