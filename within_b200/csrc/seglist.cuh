@@ -105,12 +105,11 @@ __device__ __forceinline__ FlVec<fl_w<K>()> sl_sum(const F& f, const typename F:
     return s;
 }
 
-template <class F, int K>
-__device__ __forceinline__ void seglist_body(const F& f, const SLDev& L, const int* __restrict__ skip) {
-    pdl_wait();
-    pdl_launch_dependents();
+// Block `block` of one problem.  LISTED: the short segments are those of
+// short_ids; else every short segment i is segment first + i.
+template <class F, int K, bool LISTED>
+__device__ __forceinline__ void seglist_block(const F& f, const SLDev& L, uint32_t block, uint32_t first) {
     constexpr int W = fl_w<K>(), P = fl_per_row<K>(), S = 32 / P;
-    if (skip && *skip) return;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int g = lane / P, c0 = (lane % P) * W;
@@ -120,18 +119,18 @@ __device__ __forceinline__ void seglist_body(const F& f, const SLDev& L, const i
 #pragma unroll
             for (int i = 0; i < W; ++i) s.q[i] += __shfl_xor_sync(FULL, s.q[i], o);
     };
-    if (blockIdx.x >= L.n_piece + L.medium_blocks) {   // short segments
-        const uint32_t t = (blockIdx.x - L.n_piece - L.medium_blocks) * SL_THREADS + threadIdx.x;
+    if (block >= L.n_piece + L.medium_blocks) {   // short segments
+        const uint32_t t = (block - L.n_piece - L.medium_blocks) * SL_THREADS + threadIdx.x;
         const uint32_t i = t / P;
         if (i >= L.n_short) return;
-        const uint32_t seg = __ldg(L.short_ids + i);
+        const uint32_t seg = LISTED || L.short_ids ? __ldg(L.short_ids + i) : first + i;
         const uint32_t a = __ldg(L.ptr + seg), b = __ldg(L.ptr + seg + 1);
         const typename F::Pre pre = f.pre(seg, c0);
         f.emit(seg, c0, pre, sl_sum<F, K, F::BATCH, false>(f, f.ctx(seg), a, b, 1, c0));
         return;
     }
-    if (blockIdx.x >= L.n_piece) {   // medium segments
-        const uint32_t i = (blockIdx.x - L.n_piece) * SL_WARPS + wid;
+    if (block >= L.n_piece) {   // medium segments
+        const uint32_t i = (block - L.n_piece) * SL_WARPS + wid;
         if (i >= L.n_medium) return;   // whole warps
         const uint32_t seg = __ldg(L.medium_ids + i);
         const uint32_t a = __ldg(L.ptr + seg), b = __ldg(L.ptr + seg + 1);
@@ -143,7 +142,7 @@ __device__ __forceinline__ void seglist_body(const F& f, const SLDev& L, const i
     }
     __shared__ __align__(16) double sm[SL_WARPS][K];
     __shared__ int last;
-    const SLPiece pc = L.pieces[blockIdx.x];
+    const SLPiece pc = L.pieces[block];
     FlVec<W> s = sl_sum<F, K, F::BATCH, F::PREFETCH>(f, f.ctx(pc.seg), pc.p0 + wid * S + g, pc.p1, SL_WARPS * S, c0);
     tree(s);
     if (lane < P) fl_st<W>(&sm[wid][c0], s);
@@ -154,7 +153,7 @@ __device__ __forceinline__ void seglist_body(const F& f, const SLDev& L, const i
             double t = 0.0;
 #pragma unroll
             for (int w = 0; w < SL_WARPS; ++w) t += sm[w][threadIdx.x];
-            L.part[(size_t)(L.piece_lo + blockIdx.x) * K + threadIdx.x] = t;
+            L.part[(size_t)(L.piece_lo + block) * K + threadIdx.x] = t;
             __threadfence();
         }
         __syncthreads();
@@ -181,6 +180,14 @@ __device__ __forceinline__ void seglist_body(const F& f, const SLDev& L, const i
         }
         f.emit(pc.seg, c0, f.pre(pc.seg, c0), s);
     }
+}
+
+template <class F, int K>
+__device__ __forceinline__ void seglist_body(const F& f, const SLDev& L, const int* __restrict__ skip) {
+    pdl_wait();
+    pdl_launch_dependents();
+    if (skip && *skip) return;
+    seglist_block<F, K, true>(f, L, blockIdx.x, 0);
 }
 
 template <class F, int K>
@@ -734,5 +741,40 @@ struct SlScatter {
         fl_st<W>(out + ((size_t)pr.out_off + seg) * K + c0, s);
     }
 };
+
+// Several problems of A^T u in one launch: a design of many terms has one per
+// term and column, most of them a few microseconds of work, and a launch each
+// cost more than the sums: solves of one column with eight terms of 2,000 levels on
+// 20,000 rows 1.67 -> 0.74 ms (20 iterations), with eight terms of 300 levels on
+// 1,000,000 rows 0.99 -> 0.75 ms (6 iterations).  A block finds its problem by its
+// index; the sums are those of a launch each, to the bit.
+constexpr int SL_GROUP = 8;   // problems of one launch: about 1.3 KB of kernel parameters
+// A problem of short segments only that fills the GPU on its own keeps its own
+// launch of k_segshort, whose blocks are eight per SM: eight terms of 100,000 levels
+// on 1,000,000 rows, 20 iterations, four columns (782 blocks each) 5.46 ms alone and
+// 5.65 grouped, one column (391 blocks each) 3.39 alone and 2.80 grouped.
+constexpr uint32_t SL_ALONE_BLOCKS = 148 * 4;
+struct SlGroup {
+    ScatterProb pr[SL_GROUP];
+    SLDev L[SL_GROUP];
+    uint32_t first[SL_GROUP];   // problems of short segments only: the first one
+    uint32_t block0[SL_GROUP];  // first block of each problem
+    int n;
+};
+
+template <int K>
+__global__ void __launch_bounds__(SL_THREADS)
+k_seggroup(const __grid_constant__ SlGroup G, const double* u, const double* sqrt_w, double* out,
+           const int* __restrict__ skip) {
+    pdl_wait();
+    pdl_launch_dependents();
+    if (skip && *skip) return;
+    int q = 0;
+#pragma unroll
+    for (int i = 1; i < SL_GROUP; ++i)
+        if (i < G.n && blockIdx.x >= G.block0[i]) q = i;
+    const SlScatter<K> f{G.pr[q], u, sqrt_w, out};
+    seglist_block<SlScatter<K>, K, false>(f, G.L[q], blockIdx.x - G.block0[q], G.first[q]);
+}
 
 }  // namespace wgpu

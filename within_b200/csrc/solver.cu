@@ -372,6 +372,25 @@ struct DevBook {
 // pieces a problem's long segments are cut into: one wave of resident blocks
 constexpr uint32_t SL_TARGET_BLOCKS = 148 * 6;
 
+// One problem's lists and the blocks it takes at K columns.
+template <int K>
+uint32_t sl_view(const DevBook& b, const SLPart& p, const uint32_t* ptr, SLDev& L) {
+    L.ptr = ptr;
+    L.short_ids = p.all_short ? nullptr : b.short_ids + p.short_off;
+    L.medium_ids = b.medium_ids + p.medium_lo;
+    L.n_short = p.n_short;
+    L.n_medium = p.medium_hi - p.medium_lo;
+    L.n_piece = p.piece_hi - p.piece_lo;
+    L.medium_blocks = (L.n_medium + SL_WARPS - 1) / SL_WARPS;
+    L.pieces = b.pieces + p.piece_lo;
+    L.piece_lo = p.piece_lo;
+    L.splits = b.splits;
+    L.part = b.part;
+    L.counters = b.counters;
+    return L.n_piece + L.medium_blocks +
+           (uint32_t)(((uint64_t)p.n_short * fl_per_row<K>() + SL_THREADS - 1) / SL_THREADS);
+}
+
 template <class F, int K>
 void launch_sl(const F& f, const DevBook& b, const SLPart& p, const uint32_t* ptr, const int* skip, cudaStream_t st) {
     if (p.all_short) {
@@ -383,20 +402,7 @@ void launch_sl(const F& f, const DevBook& b, const SLPart& p, const uint32_t* pt
         return;
     }
     SLDev L;
-    L.ptr = ptr;
-    L.short_ids = b.short_ids + p.short_off;
-    L.medium_ids = b.medium_ids + p.medium_lo;
-    L.n_short = p.n_short;
-    L.n_medium = p.medium_hi - p.medium_lo;
-    L.n_piece = p.piece_hi - p.piece_lo;
-    L.medium_blocks = (L.n_medium + SL_WARPS - 1) / SL_WARPS;
-    L.pieces = b.pieces + p.piece_lo;
-    L.piece_lo = p.piece_lo;
-    L.splits = b.splits;
-    L.part = b.part;
-    L.counters = b.counters;
-    const uint32_t short_blocks = (uint32_t)(((uint64_t)p.n_short * fl_per_row<K>() + SL_THREADS - 1) / SL_THREADS);
-    const uint32_t grid = L.n_piece + L.medium_blocks + short_blocks;
+    const uint32_t grid = sl_view<K>(b, p, ptr, L);
     if (!grid) return;
     if constexpr (F::FULL) launch_k(k_seglist_full<F, K>, grid, SL_THREADS, 0, st, f, L, skip);
     else launch_k(k_seglist<F, K>, grid, SL_THREADS, 0, st, f, L, skip);
@@ -1767,9 +1773,39 @@ void rowsweep_rest(within_solver& s, within_solver::RowSweepK& rk, const T* u, T
     if (!rk.n_rest) return;
     if constexpr (sizeof(T) == 8) {
         if (!rk.rest_parts.empty()) {
-            for (size_t i = 0; i < rk.rest_parts.size(); ++i)
+            SlGroup G{};
+            uint32_t blocks = 0;
+            size_t at = 0;   // the group's first problem
+            auto alone = [&](size_t i) {
                 launch_sl<SlScatter<K>, K>({rk.rest_host[i], u, s.op.sqrt_w, out}, rk.rest_book, rk.rest_parts[i],
                                            rk.rest_host[i].seg_ptr, skip, st);
+            };
+            auto flush = [&] {
+                if (G.n == 1) alone(at);
+                else if (blocks) {
+                    launch_k(k_seggroup<K>, blocks, SL_THREADS, 0, st, G, u, s.op.sqrt_w, out, skip);
+                    ++g_launches;
+                }
+                G.n = 0;
+                blocks = 0;
+            };
+            for (size_t i = 0; i < rk.rest_parts.size(); ++i) {
+                SLDev L;
+                const uint32_t b = sl_view<K>(rk.rest_book, rk.rest_parts[i], rk.rest_host[i].seg_ptr, L);
+                if (rk.rest_parts[i].all_short && b > SL_ALONE_BLOCKS) {
+                    alone(i);
+                    continue;
+                }
+                if (G.n == SL_GROUP) flush();
+                if (G.n == 0) at = i;
+                G.pr[G.n] = rk.rest_host[i];
+                G.L[G.n] = L;
+                G.first[G.n] = rk.rest_parts[i].first;
+                G.block0[G.n] = blocks;
+                blocks += b;
+                ++G.n;
+            }
+            if (G.n) flush();
             return;
         }
         ScatterF<K, 0> f{rk.rest_probs, u, s.op.sqrt_w, out, nullptr};
