@@ -675,8 +675,12 @@ bool use_lists(const Tuning& t) {
 // The suffix of rounds that k_rounds takes: each of them has to cost one block
 // less than a launch of its own.  A pass takes about 0.9 us and the block's
 // copies run at about 100 GB/s; a round's own launch takes 4.5 to 6.5 us
-// whatever its size.  The column's reduced vector, the
-// pass list and the stages have to fit in shared memory.
+// whatever its size.  The column's reduced vector, the direction's
+// pass list and the stages have to fit in shared memory: at most about 9,200
+// reduced unknowns.  Longer ones keep a launch per round; the tile engines'
+// single-block kernel for a tail of short rounds is no better (20,000 kept levels
+// in seven rounds, 20 iterations: 2.57 ms with it and 1.96 without at one
+// column, 6.99 and 3.38 at eight).
 constexpr size_t RP_SMEM_CAP = 220 * 1024;
 void plan_narrow_rounds(SchwarzUser& U, const SchwarzHost& H) {
     auto& L = U.lists;
@@ -696,7 +700,7 @@ void plan_narrow_rounds(SchwarzUser& U, const SchwarzHost& H) {
     };
     uint32_t lo = nr;
     size_t nf = 0, nb = 0;
-    while (lo > 0 && bytes(nf + nb) <= RP_SMEM_CAP) {
+    while (lo > 0 && bytes(std::max(nf, nb)) <= RP_SMEM_CAP) {
         // (a round this large is not worth packing to find out)
         if (H.fwd_round_ptr[lo] - H.fwd_round_ptr[lo - 1] > 16 * RP_WARPS * RP_SLICE) break;
         NarrowRounds f, b;
