@@ -916,15 +916,19 @@ __device__ __forceinline__ void givens(double a, double b, double& c, double& s,
     }
 }
 
-// Whether the device has raised an error in this solve; one that a wait outside
-// the solve's own word left (werr: the solver's) is taken over.  It ends every
-// column, so that no later kernel of the loop runs on vectors a failed one left
-// unwritten or waits out its own limit.  One thread.
-__device__ __forceinline__ int device_error(Ctl* ctl, const int* werr) {
-    const int e = *(const volatile int*)werr;
-    if (e) atomicCAS(&ctl->err, 0, e);
-    return *(volatile int*)&ctl->err != 0 ? 1 : 0;
-}
+// An error that earlier kernels of the solve have raised: in the solve's own word,
+// or in the solver's (werr: a timed-out wait), which end() takes over.  It ends
+// every column, so that no later kernel of the loop runs on vectors a failed one
+// left unwritten or waits out its own limit.  Read at the kernel's start, beside
+// its other loads: two loads in the last block's closing thread cost 0.5 us.
+struct DeviceError {
+    int own, wait;
+    __device__ __forceinline__ DeviceError(const Ctl* ctl, const int* werr) : own(ctl->err), wait(*werr) {}
+    __device__ __forceinline__ int end(Ctl* ctl) const {
+        if (wait) atomicCAS(&ctl->err, 0, wait);
+        return (own | wait) != 0 ? 1 : 0;
+    }
+};
 
 // One column of k_alpha_step from its sums <v, p~>, <v, v> and <p~, p~>:
 // alpha with the indefinite-M check, the recurrences, the stopping tests.
@@ -1025,6 +1029,7 @@ k_alpha_step(uint32_t n, const double* __restrict__ v, const double* __restrict_
     pdl_wait();
     pdl_launch_dependents();
     if (ctl->all_done) return;
+    const DeviceError error(ctl, werr);
     constexpr int W = fl_w<K>();
     const size_t total = (size_t)n * fl_per_row<K>();
     const size_t e0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
@@ -1059,7 +1064,7 @@ k_alpha_step(uint32_t n, const double* __restrict__ v, const double* __restrict_
         int all = 1;
         for (int k = 0; k < K; ++k) all &= col_done[k];
         ctl->k5_skip = 0;
-        ctl->all_done = all | device_error(ctl, werr);
+        ctl->all_done = all | error.end(ctl);
     }
 }
 
@@ -1462,6 +1467,7 @@ k_alpha_init(uint32_t n, const double* __restrict__ v, const double* __restrict_
              ColState* st_other, Ctl* ctl, const int* werr, double* partials, unsigned* counter) {
     pdl_wait();
     pdl_launch_dependents();
+    const DeviceError error(ctl, werr);
     constexpr int W = fl_w<K>(), P = fl_per_row<K>();
     const size_t total = (size_t)n * P;
     const size_t e0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
@@ -1518,7 +1524,7 @@ k_alpha_init(uint32_t n, const double* __restrict__ v, const double* __restrict_
         st_other[k] = s;
         all = all && s.done;
     }
-    ctl->all_done = (all ? 1 : 0) | device_error(ctl, werr);
+    ctl->all_done = (all ? 1 : 0) | error.end(ctl);
     ctl->k5_skip = 0;
 }
 
