@@ -170,6 +170,12 @@ void within_tuning_default(within_tuning* t);
 int within_solver_new_tuned(const within_design* design, const double* weights,
                             const within_precond_config* cfg, const within_preconditioner* prebuilt,
                             int32_t device, const within_tuning* tuning, within_solver** out);
+/* within_solver_new_tuned (tuning NULL: the defaults) for a solver that starts at a precision other than
+ * FP64: what is prepared at construction is that precision's.  within_solver_set_precision changes it. */
+int within_solver_new_precision(const within_design* design, const double* weights,
+                                const within_precond_config* cfg, const within_preconditioner* prebuilt,
+                                int32_t device, const within_tuning* tuning, int32_t precision,
+                                within_solver** out);
 void within_solver_free(within_solver* s);
 uint64_t within_solver_n_obs(const within_solver* s);
 uint64_t within_solver_n_dofs(const within_solver* s);

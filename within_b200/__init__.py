@@ -479,7 +479,11 @@ class Solver:
         tn = _tuning_struct(tuning, design, w)
         self.tuning = None if tn is None else {f: getattr(tn, f) for f, _ in _ffi.TuningC._fields_}
         h = C.c_void_p()
-        if tn is None:
+        if precision == "mixed":   # its plans, not FP64's, are prepared at construction
+            _ffi.check(L.within_solver_new_precision(d.h, _ffi.ptr(w), None if cfg is None else C.byref(cfg), prebuilt,
+                                                     device, None if tn is None else C.byref(tn),
+                                                     _ffi.PRECISION_MIXED, C.byref(h)))
+        elif tn is None:
             _ffi.check(L.within_solver_new(d.h, _ffi.ptr(w), None if cfg is None else C.byref(cfg),
                                            prebuilt, device, C.byref(h)))
         else:

@@ -122,6 +122,7 @@ _SIGNATURES = [
     ("within_preconditioner_stats", C.c_int, [P, P]),
     ("within_tuning_default", None, [P]),
     ("within_solver_new_tuned", C.c_int, [P, P, P, P, C.c_int32, P, P]),
+    ("within_solver_new_precision", C.c_int, [P, P, P, P, C.c_int32, P, C.c_int32, P]),
     ("within_solver_solve_batch_device_ext", C.c_int, [P, P, U64, P, P, P, P, P, P, P]),
     ("within_preconditioner_serialize", C.c_int, [P, P, U64, P]),
     ("within_preconditioner_deserialize", C.c_int, [P, U64, C.c_int32, P]),

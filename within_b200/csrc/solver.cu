@@ -754,6 +754,7 @@ void plan_narrow_rounds(SchwarzUser& U, const SchwarzHost& H) {
 void ensure_lists(SchwarzUser& U, const within_preconditioner& P) {
     auto& L = U.lists;
     if (L.ready) return;
+    PhaseTrace pt("segment lists and narrow rounds (FP64 applies)");
     const SchwarzHost& H = P.host;
     SegBook b;
     auto whole = [&](const std::vector<uint32_t>& ptr) {
@@ -782,6 +783,7 @@ void ensure_lists(SchwarzUser& U, const within_preconditioner& P) {
 void ensure_tile_plans(SchwarzUser& U, const within_preconditioner& P, int K) {
     KPlans& kp = U.kp[kidx(K)];
     if (kp.plans) return;
+    PhaseTrace pt("tile and range plans of a column bucket");
     const SchwarzHost& H = P.host;
     Arena& A = U.arena;
     const int T = plan_tile(K, false);
@@ -908,9 +910,10 @@ KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K
     return kp;
 }
 
-// FP32 work vectors of one user (allocated outside any stream capture).
+// Plans and FP32 work vectors of one user (allocated outside any stream
+// capture).  The FP32 applies read neither the lists nor the FP64 vectors.
 SchwarzWorkT<float>& schwarz_user_work_f(SchwarzUser& U, const within_preconditioner& P, int K) {
-    KPlans& kp = schwarz_user_plans(U, P, K);
+    KPlans& kp = U.kp[kidx(K)];
     ensure_tile_plans(U, P, K);
     if (!kp.wf.rl) {
         const SchwarzHost& H = P.host;
@@ -932,16 +935,16 @@ SchwarzWorkT<float>& schwarz_user_work_f(SchwarzUser& U, const within_preconditi
 template <int K, class T = double>
 void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, const int* skip,
                    cudaStream_t st, const int* keep = nullptr) {
-    KPlans& kp = schwarz_user_plans(U, P, K);
     SchwarzDevT<T> S;
     SchwarzWorkT<T>* w;
     if constexpr (sizeof(T) == 8) {
         S = P.dev_const;
-        w = &kp.w;
+        w = &schwarz_user_plans(U, P, K).w;
     } else {
         S = P.dev_const_f;
         w = &schwarz_user_work_f(U, P, K);
     }
+    const KPlans& kp = U.kp[kidx(K)];
     S.rl = w->rl;
     S.sl = w->sl;
     S.rb = w->rb;
@@ -1146,10 +1149,14 @@ struct within_solver {
         bool cs = false;
         CsTerms cs_terms{};
         size_t cs_smem = 0;
+        std::vector<int> cls;                          // term classes, for rsw_scan
+        std::vector<uint64_t> n_runs;
+        std::vector<std::vector<uint32_t>> scan_heads;   // run heads per range of rsw_scan, by run term
     } rsw[4];
-    // the scan sweep's ranges for the FP32 normal operator where rsw is cut
-    // for the column-lane sweep (built for mixed precision only; run sums shared)
-    RowSweepK rsw_f[4];
+    // the scan sweep's ranges where rsw is cut for the column-lane or the staged
+    // sweep (run sums shared; mixed precision only): the FP32 normal operator, and
+    // at one column the FP64 residual
+    RowSweepK rsw_scan[4];
     std::vector<BackTerm> back;   // slope terms' back-transform (x leaves the whitened basis)
     int* sweep_err = nullptr;   // device flag of a timed-out wait in a sweep outside the LSMR loop
     // per column bucket, the LSMR step's operator path:
@@ -1412,11 +1419,55 @@ void ensure_rest_plan(within_solver& s, within_solver::RowSweepK& rk) {
     rk.rest_plan = true;
 }
 
+// Run heads of every range of rpr rows (cnt) and, where rpr2 is not zero, of every
+// range of rpr2 rows (cnt2), in one pass over the codes.
+void run_heads(const uint32_t* codes, uint64_t n, uint64_t rpr, std::vector<uint32_t>& cnt, uint64_t rpr2,
+               std::vector<uint32_t>& cnt2) {
+    std::vector<uint64_t> at;   // starts of the pieces between the boundaries of both cuts
+    at.reserve(cnt.size() + cnt2.size() + 1);
+    uint64_t a = 0, b = 0;
+    while (std::min(a, b) < n) {
+        const uint64_t i = std::min(a, b);
+        at.push_back(i);
+        if (a == i) a += rpr;
+        if (b == i) b = rpr2 ? b + rpr2 : UINT64_MAX;
+    }
+    at.push_back(n);
+    const size_t np = at.size() - 1;
+    std::vector<uint32_t> c(np, 0);
+    par_for_each((np + 63) / 64, [&](size_t blk) {
+        for (size_t q = blk * 64; q < std::min(np, (blk + 1) * 64); ++q) {
+            uint32_t h = 0;
+            for (uint64_t i = at[q]; i < at[q + 1]; ++i) h += (i == 0 || codes[i] != codes[i - 1]) ? 1u : 0u;
+            c[q] = h;
+        }
+    });
+    for (size_t q = 0; q < np; ++q) {
+        cnt[at[q] / rpr] += c[q];
+        if (rpr2) cnt2[at[q] / rpr2] += c[q];
+    }
+}
+
+// Rows per range and blocks of a sweep on at most `grid` blocks of `per_block`
+// ranges each, cut at multiples of `ch` rows: only the blocks whose ranges hold rows.
+struct SweepCut {
+    uint64_t rpr, ranges;
+    int grid;
+};
+SweepCut cut_rows(uint64_t n, int grid, uint64_t per_block, uint64_t ch, uint64_t min_range) {
+    const uint64_t G = (uint64_t)grid * per_block;
+    SweepCut c;
+    c.rpr = std::max<uint64_t>(min_range, ((n + G - 1) / G + ch - 1) / ch * ch);
+    c.grid = (int)std::min<uint64_t>((uint64_t)grid, (n + c.rpr * per_block - 1) / (c.rpr * per_block));
+    c.ranges = (uint64_t)c.grid * per_block;
+    return c;
+}
+
 // Classifies the terms for the warp-range row sweep and builds its tables
 // (rowsweep.cuh): range bases of the run ordinals, the crossing-run fix-ups,
 // the level-sorted run combines and the remaining full-resolution terms.
-// share: only the scan sweep's ranges and partials are built (no column-lane
-// sweep, no combines), with the run sums of `share`.
+// share: only the scan sweep's ranges and partials are built (no column-lane or
+// staged sweep, no combines), with the run sums of `share`.
 template <int K>
 void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within_solver::RowSweepK* share) {
     const HostDesign& D = s.design;
@@ -1426,9 +1477,14 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
     const int Q = (int)D.terms.size();
     // term classes: hist (few coefficients), run (sorted, or few runs), rest
     enum { CLS_REST = 0, CLS_RUN = 1, CLS_HIST = 2 };
-    std::vector<int> cls(Q, CLS_REST);
-    std::vector<uint64_t> n_runs(Q, 0);
-    {
+    std::vector<int>& cls = rk.cls;
+    std::vector<uint64_t>& n_runs = rk.n_runs;
+    if (share) {
+        cls = share->cls;
+        n_runs = share->n_runs;
+    } else {
+        cls.assign(Q, CLS_REST);
+        n_runs.assign(Q, 0);
         int nh = 0, nr = 0, nbk = 0;
         for (int t = 0; t < Q; ++t) {
             const Term& T = D.terms[t];
@@ -1469,7 +1525,7 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
             one_slope = one_slope && D.terms[t].cols.size() <= 2;
             if (cls[t] == CLS_HIST) nbk += (int)(D.terms[t].n_levels * D.terms[t].cols.size());
         }
-        const bool ok = K == 1 && (simple || one_slope) && Q <= TS_MAXQ && nrun >= 1 && s.schwarz.tuning.staged;
+        const bool ok = K == 1 && !share && (simple || one_slope) && Q <= TS_MAXQ && nrun >= 1 && s.schwarz.tuning.staged;
         const size_t sm = simple ? ts_smem_bytes<K>(nbk, nhist, Q, s.op.sqrt_w != nullptr)
                                  : ts_ring_offset<K>(nbk, nhist);
         if (ok && sm <= TS_SMEM_CAP) {
@@ -1489,8 +1545,7 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
     // the staged sweep: as many blocks per SM as its bins and rings leave room for
     rk.grid = !rk.ts ? rw_grid<K>()
                      : 148 * (rk.ts_ns == 0 && rk.ts_smem <= TS_SMEM_FULL ? TS_BLOCKS_PER_SM : 2);
-    uint64_t G = (uint64_t)rk.grid * RW_WARPS;   // ranges
-    uint64_t CH = rw_chunk<K>(), min_range = CH;
+    SweepCut cut = cut_rows(n, rk.grid, RW_WARPS, rw_chunk<K>(), rw_chunk<K>());
     // several columns of an intercept-only design of at most three terms: the
     // column-lane sweep (csweep.cuh; a third of the scan sweep's time at eight
     // columns, half at four), one range per stream, as many blocks as the rows
@@ -1504,24 +1559,20 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
                 if (cls[t] == CLS_HIST) nbk += (int)D.terms[t].n_levels;
             const uint64_t per_block = (uint64_t)CS_WARPS * cs_streams<K>();
             const uint64_t want = (n + CS_MIN_RANGE * per_block - 1) / (CS_MIN_RANGE * per_block);
-            rk.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, 148ull * cs_blocks_per_sm(nbk)));
+            cut = cut_rows(n, (int)std::max<uint64_t>(1, std::min<uint64_t>(want, 148ull * cs_blocks_per_sm(nbk))),
+                           per_block, CS_ROWS, CS_MIN_RANGE);
             rk.cs_smem = cs_smem_bytes(nbk);
             rk.cs_terms.nq = Q;
-            G = (uint64_t)rk.grid * per_block;
-            CH = CS_ROWS;
-            min_range = CS_MIN_RANGE;
         }
     }
-    uint64_t rpr = (n + G - 1) / G;
-    rpr = std::max<uint64_t>(min_range, (rpr + CH - 1) / CH * CH);
+    // (on 2,003 rows the last block of a full grid added 444 blocks' bins for 31 of the sweep's 34 us)
+    rk.grid = cut.grid;
+    const uint64_t rpr = cut.rpr, G = cut.ranges;
     rp.rows_per_range = (uint32_t)rpr;
-    // only the blocks whose ranges hold rows: on 2,003 rows the last block of a
-    // full grid added 444 blocks' bins for 31 of the sweep's 34 us
-    {
-        const uint64_t per_block = rpr * (G / (uint64_t)rk.grid);
-        rk.grid = (int)std::min<uint64_t>((uint64_t)rk.grid, (n + per_block - 1) / per_block);
-        G = (uint64_t)rk.grid * (per_block / rpr);
-    }
+    // a mixed solver needs the scan sweep's ranges as well: their run heads in the same pass
+    SweepCut scan{};
+    if (!share && (rk.cs || rk.ts) && s.precision == WITHIN_PRECISION_MIXED)
+        scan = cut_rows(n, rw_grid<K>(), RW_WARPS, rw_chunk<K>(), rw_chunk<K>());
     std::vector<RwFix> fixes;
     size_t first_prob = 0;
     for (int t = 0; t < Q; ++t) {
@@ -1541,18 +1592,18 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
         }
         if (cls[t] == CLS_RUN) {
             // run heads per range
-            std::vector<uint32_t> cnt(G, 0);
+            std::vector<uint32_t> cnt;
             const uint64_t runs = n_runs[t];
-            par_for_each((size_t)((G + 63) / 64), [&](size_t b) {
-                for (uint64_t g = b * 64; g < std::min<uint64_t>(G, (b + 1) * 64); ++g) {
-                    const uint64_t i0 = g * rpr, i1 = std::min<uint64_t>(n, i0 + rpr);
-                    uint32_t c = 0;
-                    for (uint64_t i = i0; i < i1; ++i) c += (i == 0 || codes[i] != codes[i - 1]) ? 1u : 0u;
-                    cnt[g] = c;
-                }
-            });
-            const bool sorted_runs = T.sorted != 0;
             const int j = rp.n_run++;
+            if (share && !share->scan_heads.empty()) {
+                cnt = share->scan_heads[j];
+            } else {
+                std::vector<uint32_t> scan_cnt(scan.ranges, 0);
+                cnt.assign(G, 0);
+                run_heads(codes.data(), n, rpr, cnt, scan.rpr, scan_cnt);
+                if (scan.rpr) rk.scan_heads.push_back(std::move(scan_cnt));
+            }
+            const bool sorted_runs = T.sorted != 0;
             if (rk.cs) {
                 rk.cs_terms.cls[t] = 1;
                 rk.cs_terms.slot[t] = j;
@@ -1692,17 +1743,25 @@ within_solver::RowSweepK& ensure_rowsweep(within_solver& s) {
     return rk;
 }
 
-// the sweep plan of the FP32 normal operator
+// the plan of the scan sweep (k_rowsweep)
 template <int K>
-within_solver::RowSweepK& rowsweep_f(within_solver& s) {
-    return s.rsw[kidx(K)].cs ? s.rsw_f[kidx(K)] : s.rsw[kidx(K)];
+within_solver::RowSweepK& ensure_scan(within_solver& s) {
+    auto& rk = ensure_rowsweep<K>(s);
+    if (!rk.cs && !rk.ts) return rk;
+    auto& sc = s.rsw_scan[kidx(K)];
+    if (!sc.ready) {
+        build_rowsweep<K>(s, sc, &rk);
+        rk.scan_heads.clear();
+        rk.scan_heads.shrink_to_fit();
+    }
+    return sc;
 }
 
 // FP32 loading columns in the rest problems (mixed-precision inner solve)
 template <int K>
 void ensure_rowsweep_f(within_solver& s) {
     auto& rk = ensure_rowsweep<K>(s);
-    if (rk.cs && !s.rsw_f[kidx(K)].ready) build_rowsweep<K>(s, s.rsw_f[kidx(K)], &rk);
+    ensure_scan<K>(s);
     if (rk.rest_probs_f || !rk.n_rest) return;
     ensure_rest_plan<K>(s, rk);
     std::vector<ScatterProb> pf = rk.rest_host;
@@ -1854,10 +1913,17 @@ within_solver::Work& work_buffers(within_solver& s, int K) {
 
 within_solver::Work& ensure_work(within_solver& s, int K) {
     auto& w = s.work[kidx(K)];
-    if (w.ready) return w;
+    // the applies' plans are those of the solver's precision, which may change between calls
+    const bool schwarz = s.precond && s.precond->kind == 1, mixed = s.precision == WITHIN_PRECISION_MIXED;
+    const KPlans& kp = s.schwarz.kp[kidx(K)];
+    if (w.ready && (!schwarz || (mixed ? kp.plans && kp.wf.rl : kp.ready))) return w;
     PhaseTrace pt("first use of a column bucket: workspaces and plans");
+    if (schwarz) {
+        if (mixed) schwarz_user_work_f(s.schwarz, *s.precond, K);
+        else schwarz_user_plans(s.schwarz, *s.precond, K);
+    }
+    if (w.ready) return w;
     work_buffers(s, K);
-    if (s.precond && s.precond->kind == 1) schwarz_user_plans(s.schwarz, *s.precond, K);
     ensure_scatter(s, K);
     // Path choice per column count, fixed per process so results stay bitwise
     // reproducible.  WITHIN_SWEEP=0 forces the gather + scatter path.
@@ -2199,7 +2265,7 @@ void cg_iteration(within_solver& s, within_solver::Work& w, within_solver::Mixed
     const int* skip = &m.ctl->all_done;
     if (s.path[kidx(K)] == 2) {
         auto& rk = s.rsw[kidx(K)];
-        launch_rowsweep<K, 2, float>(s, rowsweep_f<K>(s), s.op_f, m.q, m.p, m.t, nullptr, m.ctl, skip,
+        launch_rowsweep<K, 2, float>(s, ensure_scan<K>(s), s.op_f, m.q, m.p, m.t, nullptr, m.ctl, skip,
                                      rk.rest_needs_rows ? 1 : 0, st);
         rowsweep_rest<K, float>(s, rk, m.t, m.q, skip, st);
     } else {
@@ -2254,7 +2320,8 @@ void mixed_pre(within_solver& s, within_solver::Work& w, within_solver::MixedWor
     const uint32_t nd = (uint32_t)s.n_dofs;
     if (s.path[kidx(K)] == 2) {   // r = b - A x, ||r||^2 and g = A^T r in one row sweep
         auto& rk = s.rsw[kidx(K)];
-        launch_rowsweep<K, 3, double>(s, rk, s.op, m.g64, m.x64, m.r64, nullptr, nullptr, nullptr,
+        // several columns: the column-lane sweep; one: the scan sweep
+        launch_rowsweep<K, 3, double>(s, rk.cs ? rk : ensure_scan<K>(s), s.op, m.g64, m.x64, m.r64, nullptr, nullptr, nullptr,
                                       rk.rest_needs_rows ? 1 : 0, st, w.b, &m.st[0].rnorm2,
                                       (int)(sizeof(CgCol) / sizeof(double)));
         rowsweep_rest<K, double>(s, rk, m.r64, m.g64, nullptr, st);
@@ -2541,12 +2608,13 @@ int guarded(F f) {
 // upload; solver sets, which solve column batches, leave them to first use.
 within_solver* make_solver(const within_design* d, const double* weights, const within_precond_config* cfg,
                            const within_preconditioner* prebuilt, int device, const within_tuning* tuning = nullptr,
-                           bool prepare_single = true) {
+                           bool prepare_single = true, int precision = WITHIN_PRECISION_FP64) {
     if (!d) throw WError(ERR_INVALID, "design is NULL");
     if (device < 0) CK(cudaGetDevice(&device));
     set_device(device);
     auto s = std::make_unique<within_solver>();
     s->device = device;
+    s->precision = precision;
     CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     s->sweep_err = s->arena.alloc<int>(1);
     s->schwarz.tuning = resolve_tuning(tuning);
@@ -2797,7 +2865,8 @@ within_solver* make_solver(const within_design* d, const double* weights, const 
                         plans = std::thread([&] {
                             try {
                                 set_device(device);
-                                schwarz_user_plans(s->schwarz, *P, 1);
+                                if (precision == WITHIN_PRECISION_MIXED) schwarz_user_work_f(s->schwarz, *P, 1);
+                                else schwarz_user_plans(s->schwarz, *P, 1);
                             } catch (...) {
                                 plan_err = std::current_exception();
                             }
@@ -3125,6 +3194,19 @@ int within_solver_new_tuned(const within_design* design, const double* weights, 
         if (tuning && !(tuning->core_min_frac >= 0.0 && tuning->core_min_frac <= 1.0))
             throw WError(ERR_INVALID, "tuning: core_min_frac must lie in [0, 1]");
         *out = make_solver(design, weights, cfg, prebuilt, device, tuning);
+    });
+}
+
+int within_solver_new_precision(const within_design* design, const double* weights, const within_precond_config* cfg,
+                                const within_preconditioner* prebuilt, int32_t device, const within_tuning* tuning,
+                                int32_t precision, within_solver** out) {
+    *out = nullptr;
+    return guarded([&] {
+        if (precision != WITHIN_PRECISION_FP64 && precision != WITHIN_PRECISION_MIXED)
+            throw WError(ERR_INVALID, "unknown precision " + std::to_string(precision));
+        if (tuning && !(tuning->core_min_frac >= 0.0 && tuning->core_min_frac <= 1.0))
+            throw WError(ERR_INVALID, "tuning: core_min_frac must lie in [0, 1]");
+        *out = make_solver(design, weights, cfg, prebuilt, device, tuning, true, precision);
     });
 }
 
