@@ -1470,6 +1470,7 @@ SweepCut cut_rows(uint64_t n, int grid, uint64_t per_block, uint64_t ch, uint64_
 // staged sweep, no combines), with the run sums of `share`.
 template <int K>
 void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within_solver::RowSweepK* share) {
+    PhaseTrace pt(share ? "scan sweep ranges of a column bucket" : "row sweep plan of a column bucket");
     const HostDesign& D = s.design;
     const uint64_t n = D.n_obs;
     Arena& A = s.arena;
@@ -3405,6 +3406,13 @@ int within_solver_operator_apply_adjoint(within_solver* s, const double* u_dev, 
         const int path = env_path(2);
         if (path == 2) {
             auto& rk = ensure_rowsweep<1>(*s);
+            // the sweeps read u by 16-byte accesses and bulk copies: a vector that starts
+            // between 16-byte boundaries (a slice) goes through the solver's own workspace
+            if (((uintptr_t)u_dev & 15) != 0) {
+                auto& w = work_buffers(*s, 1);
+                CK(cudaMemcpyAsync(w.u, u_dev, s->n_obs * sizeof(double), cudaMemcpyDeviceToDevice, st));
+                u_dev = w.u;
+            }
             CK(cudaMemsetAsync(y_dev, 0, s->n_dofs * sizeof(double), st));   // levels no row reaches stay 0
             launch_rowsweep<1, 0, double>(*s, rk, s->op, y_dev, nullptr, const_cast<double*>(u_dev), nullptr,
                                           nullptr, nullptr, 0, st);
