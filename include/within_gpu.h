@@ -95,7 +95,8 @@ typedef struct {
     int32_t converged;
     uint64_t iterations;          /* LSMR iterations (summed over refinement sweeps) */
     double residual;              /* relative normal-equation residual estimate */
-    double time_total, time_setup, time_solve;   /* seconds */
+    double time_total, time_setup, time_solve;   /* seconds: the call; until its right-hand sides are loaded;
+                                                    the iteration (the rest: demeaning and results) */
 } within_solve_stats;
 
 typedef struct within_design within_design;

@@ -12,6 +12,7 @@
 #include <climits>
 #include <cstdint>
 
+#include "bulk.cuh"
 #include "segreduce.cuh"
 #include "segsweep.cuh"
 
@@ -61,7 +62,8 @@ struct Ctl {
     int bodies_left;  // device-side graph loop: bodies (2 iterations each) still allowed
     int bodies_run;   // device-side graph loop: bodies executed
     int outer;        // mixed precision: refinement steps taken
-    int pad[2];
+    // global timer (ns) as the solve starts on its loaded right-hand side, and after the loop's last body
+    unsigned long long t_begin, t_end;
 };
 
 // End of one body (two LSMR iterations) of the device-side graph loop: run
@@ -71,7 +73,15 @@ __global__ void k_loop_cond(Ctl* ctl, cudaGraphConditionalHandle h) {
     const int left = ctl->bodies_left - 1;
     ctl->bodies_left = left;
     ctl->bodies_run += 1;
+    ctl->t_end = global_ns();
     cudaGraphSetConditional(h, (!ctl->all_done && !ctl->err && left > 0) ? 1u : 0u);
+}
+
+// The end of a loop that the host drives.
+__global__ void k_loop_end(Ctl* ctl) {
+    pdl_wait();
+    pdl_launch_dependents();
+    ctl->t_end = global_ns();
 }
 
 // LsmrStopReason (lsmr.rs:54-73), same order
@@ -1280,6 +1290,7 @@ k_norm_b(uint32_t n, const double* __restrict__ b, const double* bmax, ColState*
          int warm = 0, int stale_window = 0, double stale_thr = 0.0) {
     pdl_wait();
     pdl_launch_dependents();
+    if (!warm && blockIdx.x == 0 && threadIdx.x == 0) ctl->t_begin = global_ns();
     constexpr int W = fl_w<K>(), P = fl_per_row<K>();
     const size_t total = (size_t)n * P;
     const size_t e0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;

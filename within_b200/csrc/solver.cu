@@ -1055,8 +1055,16 @@ struct SolveState {
     ColState st[16];
     Ctl ctl;
     int nonfinite;
-    int sweep_err;   // copied from the solver's flag before the read
+    int sweep_err;   // copied from the solver's flag by k_solve_end
+    unsigned long long t_fin;   // global timer (ns) after the results
 };
+
+__global__ void k_solve_end(SolveState* s, const int* sweep_err) {
+    pdl_wait();
+    pdl_launch_dependents();
+    s->sweep_err = *sweep_err;
+    s->t_fin = global_ns();
+}
 
 // ---------------------------------------------------------------------------
 struct within_solver {
@@ -2076,7 +2084,6 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
         launch_k(k_load_x0<K>, grid_for(nd, 256, 148 * 8), 256, 0, st, nd, k_used, ext.x0, w.x0, w.nonfinite);
         ++g_launches;
     }
-    const double t_solve0 = now_s();
     launch_k(k_norm_b<K>, fl_grid<K>(n), RED_THREADS, 0, st, n, w.b, w.bmax, w.st, tol, (long long)maxiter, k_used,
                                                   w.ctl, w.partials, w.counter, w.nonfinite, 0,
                                                   (int)ext.stale_window, ext.stale_threshold);
@@ -2138,6 +2145,8 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
         uint64_t left = (maxiter + 2 - done_iters + 1) / 2;
         burst = std::max<uint64_t>(1, std::min(burst, left));
     }
+    launch_k(k_loop_end, 1, 1, 0, st, w.ctl);
+    ++g_launches;
     }
     // results
     if (ext.x0) {
@@ -2160,7 +2169,8 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
     }
     ColState fin[8];
     SolveState out;
-    CK(cudaMemcpyAsync(&w.state->sweep_err, s.sweep_err, sizeof(int), cudaMemcpyDeviceToDevice, st));
+    launch_k(k_solve_end, 1, 1, 0, st, w.state, s.sweep_err);
+    ++g_launches;
     CK(cudaMemcpyAsync(&out, w.state, sizeof(SolveState), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (device_loop) g_launches += (uint64_t)out.ctl.bodies_run * w.graph_iters;
@@ -2175,7 +2185,11 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
     if (out.ctl.err == ERR_WARM_NONFINITE)
         throw WError(ERR_INVALID, "warm-start residual b - A x0 has a non-finite norm");
     if (out.sweep_err) throw WError(ERR_CUDA, WAIT_TIMEOUT_TEXT);
-    const double t_solve1 = now_s();
+    // time_setup: up to the loaded right-hand side; time_solve: from there to the loop's end; the rest of
+    // time_total: demeaning and the results.  The host waits once, so the device's stamps divide the time.
+    const double t_sync = now_s();
+    const double solve_s = 1e-9 * (double)(out.ctl.t_end - out.ctl.t_begin);
+    const double setup_s = std::max(0.0, t_sync - t_setup0 - 1e-9 * (double)(out.t_fin - out.ctl.t_begin));
     // the state parity after the loop is whichever buffer was written last:
     // both buffers hold identical done states for finished columns, so read
     // the one with the larger iteration count.
@@ -2193,8 +2207,8 @@ void run_lsmr(within_solver& s, within_solver::Work& w, const double* Y, uint32_
             o.iterations = (uint64_t)c.itn;
             o.residual = (c.stop == STOP_ZERO_RHS || c.stop == STOP_INIT_ZERO || c.stop == STOP_WARM_EXACT)
                              ? 0.0 : fabs(c.zeta_bar) / c.zeta0;
-            o.time_setup = t_solve0 - t_setup0;
-            o.time_solve = t_solve1 - t_solve0;
+            o.time_setup = setup_s;
+            o.time_solve = solve_s;
             o.time_total = t_end - t_setup0;
         }
 }
