@@ -15,6 +15,12 @@ namespace wgpu {
 constexpr uint32_t SL_SHORT = 32;
 constexpr uint32_t SL_MEDIUM = 512;
 
+// The lists' kernels step through positions in 32 bits, at most eight batches of
+// a block's 256 lanes beyond a segment's end: a plan whose positions come closer
+// to 2^32 would wrap around there, and stays on the tile and range engines.
+constexpr uint32_t SL_STEP = 8 * 256;
+constexpr bool sl_fits(uint64_t positions) { return positions + 2 * SL_STEP <= UINT32_MAX; }
+
 struct SLPiece {
     uint32_t seg, p0, p1;   // positions [p0, p1) of segment seg
     int32_t split;          // split id when the segment has several pieces, else -1

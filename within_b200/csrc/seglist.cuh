@@ -40,6 +40,7 @@ namespace wgpu {
 constexpr int SL_THREADS = 256;
 constexpr int SL_WARPS = SL_THREADS / 32;
 constexpr int SL_BATCH = 8;
+static_assert(SL_BATCH * SL_THREADS <= (int)SL_STEP, "a step past the end stays below the wrap");
 
 // device view of one problem's lists; blocks [0, pieces) take the pieces, then
 // the medium segments (one warp each), then the short ones

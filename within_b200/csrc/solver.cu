@@ -672,6 +672,12 @@ bool use_lists(const Tuning& t) {
     return t.warp_ranges == 1 && t.segthread && !t.vector_rows && t.wide_mean_len == UINT32_MAX;
 }
 
+// ... and whether the image's arrays are short enough for them.
+bool use_lists(const Tuning& t, const SchwarzHost& H) {
+    return use_lists(t) && sl_fits(std::max({H.glob.size(), H.ct_col.size(), H.c_col.size(), H.fwd_col.size(),
+                                             H.bwd_col.size(), H.dense_col.size(), H.core_col.size()}));
+}
+
 // The suffix of rounds that k_rounds takes: each of them has to cost one block
 // less than a launch of its own.  A pass takes about 0.9 us and the block's
 // copies run at about 100 GB/s; a round's own launch takes 4.5 to 6.5 us
@@ -895,7 +901,7 @@ KPlans& schwarz_user_plans(SchwarzUser& U, const within_preconditioner& P, int K
     if (kp.ready) return kp;
     const SchwarzHost& H = P.host;
     Arena& A = U.arena;
-    if (use_lists(U.tuning)) ensure_lists(U, P);
+    if (use_lists(U.tuning, H)) ensure_lists(U, P);
     else ensure_tile_plans(U, P, K);
     size_t nl = H.glob.size(), nr = H.n_red, ns = H.n_sub;
     kp.w.rl = A.alloc<double>(nl * K);
@@ -968,7 +974,7 @@ void schwarz_apply(within_preconditioner& P, SchwarzUser& U, const T* r, T* z, c
         ++g_launches;
     };
     if constexpr (sizeof(T) == 8) {
-        if (use_lists(U.tuning)) {
+        if (use_lists(U.tuning, P.host)) {
             const auto& L = U.lists;
             const DevBook& b = L.book;
             launch_sl<SlRestrict<K>, K>({{S}, r}, b, L.restrict_, S.loc_ptr, skip, st);
@@ -1691,7 +1697,7 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
     if (!share) rk.atu = A.alloc<double>(s.n_dofs * K);
     rk.n_rest = (uint32_t)rk.rest_host.size();
     if (rk.n_rest) {
-        if (use_lists(s.schwarz.tuning)) {
+        if (use_lists(s.schwarz.tuning) && sl_fits(n)) {
             SegBook book;
             for (const auto& lp : rk.rest_ptrs)
                 rk.rest_parts.push_back(book.add(lp.data(), 0, (uint32_t)lp.size() - 1, SL_TARGET_BLOCKS));
