@@ -20,7 +20,22 @@
 // weighted, four columns: 145 -> 76 us.  Four rows per step because each
 // stream then reads 256 consecutive bytes of u per request (with two rows the
 // same kernel took 501 us); three blocks per SM because the registers of four
-// (128 per thread) spill.
+// (128 per thread) spill.  The weighted step of four and eight columns spills all
+// the same at 168 registers (about 100 bytes a thread; weights cost 20 us of 119 at
+// eight columns).  What is left is latency at low occupancy: 12 warps per SM,
+// 18 % of the warp slots, waiting for u and for gathered coefficients (long
+// scoreboard), DRAM at 39 % with eight columns and 16 % with two.
+//
+// The private bins take 2 KB per level and block, so a histogram term of more
+// than 35 levels leaves two blocks per SM and one of more than 53 a single one,
+// and at two columns every lane walks a range of its own.  It is taken there too:
+// LSMR step of 2,000,000 rows against the scan sweep, us (weighted in brackets):
+//   bins      two columns          four columns           eight columns
+//     20   69 -> 46  (72 -> 52)  146 ->  65 (149 ->  78)  331 -> 100 (332 -> 120)
+//     35   82 -> 66  (88 -> 82)  159 -> 102 (160 -> 113)  353 -> 137 (356 -> 142)
+//     50   89 -> 72  (94 -> 88)  182 -> 111 (185 -> 131)  408 -> 143 (412 -> 175)
+//     64   95 -> 61 (100 -> 79)  203 -> 113 (205 -> 138)  447 -> 198 (448 -> 242)
+// and 1.3 to 7 times as fast on 200,000 rows.
 //
 // The ranges are those of rowsweep.cuh with one range per stream: a run that
 // crosses ranges leaves a tail partial and head partials, which k_cs_finish

@@ -9,7 +9,8 @@ namespace wgpu {
 
 // Segments of at most SL_SHORT positions are summed by one group of lanes each,
 // longer ones of at most SL_MEDIUM by one warp, the rest in pieces by blocks.
-// SL_SHORT: one batch of loads per lane covers most of the segment.  SL_MEDIUM:
+// SL_SHORT: what one group of lanes sums in a few batches of loads (eight positions
+// at a time, two in k_segshort).  SL_MEDIUM:
 // at eight columns a warp takes eight positions per step, so 512 positions are
 // eight batches of eight steps; a block would leave most of its warps idle.
 constexpr uint32_t SL_SHORT = 32;

@@ -208,7 +208,7 @@ k_seglist_full(F f, SLDev L, const int* __restrict__ skip) {
 // two or three dependent loads of so little work, so the kernel is held to 32
 // registers (eight blocks per SM) and asks for two positions at a time: C of the
 // 10,000,000-row panel (10.4 M non-zeros in rows of about five) takes 62 us with
-// one column and 146 us with eight; 236 us with eight positions at a time in 64
+// one column and 146 to 152 us over runs with eight; 236 us with eight positions at a time in 64
 // registers, 183 us with four in 40, 66 us (one column) with the values of a
 // warp's segments staged in shared memory.
 constexpr int SL_SHORT_BATCH = 2;
@@ -303,7 +303,8 @@ struct SlBase {
 template <int K>
 struct SlRestrict : SlBase<K> {
     // it streams: resident warps are worth more than loads per lane (71 -> 52 us at
-    // eight columns, 14 -> 10 at four)
+    // eight columns, 14 -> 10 at four), and than the few registers that spill for
+    // it at four and eight columns (24 bytes of stack)
     static constexpr int BATCH = 4;
     static constexpr bool PREFETCH = false, FULL = true;
     SL_TYPES;

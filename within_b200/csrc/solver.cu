@@ -1562,8 +1562,9 @@ void build_rowsweep(within_solver& s, within_solver::RowSweepK& rk, const within
                      : 148 * (rk.ts_ns == 0 && rk.ts_smem <= TS_SMEM_FULL ? TS_BLOCKS_PER_SM : 2);
     SweepCut cut = cut_rows(n, rk.grid, RW_WARPS, rw_chunk<K>(), rw_chunk<K>());
     // several columns of an intercept-only design of at most three terms: the
-    // column-lane sweep (csweep.cuh; a third of the scan sweep's time at eight
-    // columns, half at four), one range per stream, as many blocks as the rows
+    // column-lane sweep (csweep.cuh; a third to a half of the scan sweep's time at
+    // eight columns, a half to two thirds at four, 0.64 to 0.94 at two, over 12 to 64
+    // histogram bins), one range per stream, as many blocks as the rows
     // fill.  Slopes and more terms need loadings per row and codes of a fourth
     // term in registers: they stay on the scan sweep.
     if constexpr (K >= 2) {
